@@ -18,6 +18,7 @@
  * comparable job by job.
  */
 #include "mmc_internal.h"
+#include "pattern.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -99,16 +100,9 @@ namespace
                 ++nulls;
                 continue;
             }
-            ulonglong2* q = reinterpret_cast<ulonglong2*>(ptr);
-            const uint32_t n16 = bytes / 16u;
-            for(uint32_t i = 0; i < n16; ++i)
-                q[i] = make_ulonglong2(m + 2u * i, m + 2u * i + 1u);
-            for(uint32_t i = 0; i < n16; ++i)
-            {
-                const ulonglong2 v = q[i];
-                bad += (v.x != m + 2u * i) + (v.y != m + 2u * i + 1u);
-                csum += v.x ^ v.y;
-            }
+            uint32_t wrong = 0;
+            thread_pattern<1>(ptr, bytes, m, wrong, csum);
+            bad += wrong;
             dv::free<Ids>(h, ptr);
             ++pairs;
         }
@@ -264,16 +258,7 @@ __global__ void __launch_bounds__(256, 4) mmc_batch_kernel(mmc_device_handle h, 
                 ++nulls;
             else
             {
-                ulonglong2* q = reinterpret_cast<ulonglong2*>(ptr);
-                const uint32_t n16 = bytes / 16u;
-                for(uint32_t i = 0; i < n16; ++i)
-                    q[i] = make_ulonglong2(m + 2u * i, m + 2u * i + 1u);
-                for(uint32_t i = 0; i < n16; ++i)
-                {
-                    const ulonglong2 v = q[i];
-                    bad += (v.x != m + 2u * i) + (v.y != m + 2u * i + 1u);
-                    csum += v.x ^ v.y;
-                }
+                thread_pattern<1>(ptr, bytes, m, bad, csum);
                 dv::free<Ids>(h, ptr);
                 ++pairs;
             }

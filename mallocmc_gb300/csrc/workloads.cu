@@ -9,6 +9,7 @@
  * (tests/verify_heap.cpp:333-388 in the reference is the pattern).
  */
 #include "mmc_internal.h"
+#include "pattern.cuh"
 
 #include <algorithm>
 
@@ -56,83 +57,111 @@ __global__ void mmc_program_kernel(mmc_device_handle h, const uint8_t* kinds, co
 
 __global__ void mmc_store_result_kernel(const unsigned* src, int64_t* dst) { *dst = static_cast<int64_t>(*src); }
 
-constexpr uint32_t kPatternGroup = 2u; /* blocks whose read-back is in flight together */
+constexpr uint32_t kPatternRows = 4u; /* rows whose read-back is in flight together */
+
+/* The 256-byte pieces of a warp's blocks (the last of a block may be shorter). */
+struct PatternPieces
+{
+    ulonglong2 at[128u + 2u * kPatternRows]; /* {global address, its first pattern word} */
+    uint32_t units[128u + 2u * kPatternRows]; /* 2 * its 16-byte units + (handled by the other half's lanes) */
+};
 
 /* Write then verify the u64 pattern m + i of `bytes` bytes at every lane's
- * block, cooperatively: the warp walks the blocks of its lanes in turn and
- * moves 512 contiguous bytes per instruction (16 per lane), instead of each
- * lane streaming its own block 16 bytes at a time across 32 cache lines.
- * The read-back issues the first 1 KiB of kPatternGroup blocks before it
- * compares any, so their loads are in flight together. Each lane reads back
- * the 16-byte units it wrote (units lane, lane + 32, ... of every block).
- * Every lane of the warp must call it (blocks of lanes whose ptr is null are
- * skipped). Returns the pattern mismatches found in this lane's share. */
-__device__ __forceinline__ uint32_t warp_pattern(char* ptr, uint32_t bytes, uint64_t m, unsigned long long& csum)
+ * block, the warp together: 512 bytes per instruction (16 per lane) instead of
+ * each lane streaming its own block 16 bytes at a time across 32 cache lines.
+ * The blocks are cut into 256-byte pieces, listed in shared memory, and each
+ * half of the warp moves one piece per row, so a row is 0.89 full for sizes of
+ * 16 to 1024 bytes where a row of one block's bytes was 0.61, and a lane finds
+ * its address and word with two shared loads where five shuffles and a bit
+ * search were. What bounded the form that moved one block per row was
+ * instructions: 3 600 of 5 200 per warp and round of the uniform stress, now
+ * 2 500 (the launch 6.82 -> 5.05 ms); 208-byte blocks 0.90 -> 0.52 ms. What
+ * bounds it now is the chain of round trips, with half the issue slots idle;
+ * two, three or six rows in flight timed as four do. The read-back issues kPatternRows rows before it
+ * compares any; their differences are folded into one word, and counted only
+ * if it is not zero. Every lane of the warp must call it. Returns the pattern
+ * mismatches this lane saw.
+ *
+ * The checksum's lanes: unit i of a block counts for lane i % 32, so a piece
+ * that the other half of the warp moves adds to `other`, which is lane ^ 16's. */
+__device__ __forceinline__ uint32_t warp_pattern(char* ptr, uint32_t bytes, uint64_t m, unsigned long long& csum,
+                                                 unsigned long long& other, PatternPieces& pieces)
 {
     const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t half = lane >> 4, sub = lane & 15u, odd = 2u * sub + 1u;
+    const uint32_t units = ptr != nullptr ? bytes / 16u : 0u;
     uint32_t bad = 0;
-    const unsigned have = __ballot_sync(0xFFFFFFFFu, ptr != nullptr);
-    for(unsigned rest = have; rest != 0u; rest &= rest - 1u)
+    /* 1 KiB of every block per pass */
+    for(uint32_t base = 0; __any_sync(0xFFFFFFFFu, units > base); base += 64u)
     {
-        const int k = __ffs(static_cast<int>(rest)) - 1;
-        ulonglong2* q = reinterpret_cast<ulonglong2*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(ptr), k));
-        const uint32_t n16 = __shfl_sync(0xFFFFFFFFu, bytes, k) / 16u;
-        const uint64_t mk = __shfl_sync(0xFFFFFFFFu, m, k);
-        for(uint32_t i = lane; i < n16; i += 32u)
-            q[i] = make_ulonglong2(mk + 2u * i, mk + 2u * i + 1u);
-    }
-    __syncwarp();
-    for(unsigned rest = have; rest != 0u;)
-    {
-        const ulonglong2* q[kPatternGroup];
-        uint32_t n16[kPatternGroup];
-        uint64_t mk[kPatternGroup];
+        const uint32_t left = units > base ? min(units - base, 64u) : 0u;
+        const uint32_t mine = (left + 15u) / 16u;
+        uint32_t incl = mine;
 #pragma unroll
-        for(uint32_t j = 0; j < kPatternGroup; ++j)
+        for(uint32_t off = 1u; off < 32u; off <<= 1)
         {
-            const bool live = rest != 0u;
-            const int k = live ? __ffs(static_cast<int>(rest)) - 1 : 0;
-            rest &= rest - 1u;
-            q[j] = reinterpret_cast<const ulonglong2*>(
-                __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(ptr), k));
-            const uint32_t nk = __shfl_sync(0xFFFFFFFFu, bytes, k) / 16u;
-            n16[j] = live ? nk : 0u;
-            mk[j] = __shfl_sync(0xFFFFFFFFu, m, k);
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+            incl += lane >= off ? v : 0u;
         }
-        ulonglong2 v[kPatternGroup][2];
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        const uint64_t a0 = __cvta_generic_to_global(ptr) + 16u * base, m0 = m + 2u * base;
 #pragma unroll
-        for(uint32_t j = 0; j < kPatternGroup; ++j)
+        for(uint32_t j = 0; j < 4u; ++j)
+            if(j < mine)
+            {
+                const uint32_t k = incl - mine + j;
+                pieces.at[k] = make_ulonglong2(a0 + 256u * j, m0 + 32u * j);
+                pieces.units[k] = 2u * min(left - 16u * j, 16u) + ((j ^ k) & 1u);
+            }
+        if(lane < 2u * kPatternRows)
+            pieces.units[total + lane] = 0u; /* the last rows' missing pieces */
+        __syncwarp();
+#pragma unroll 1
+        for(uint32_t k = half; k < total; k += 2u * kPatternRows)
         {
 #pragma unroll
-            for(uint32_t u = 0; u < 2u; ++u)
+            for(uint32_t r = 0; r < kPatternRows; ++r)
             {
-                const uint32_t i = lane + 32u * u;
-                v[j][u] = i < n16[j] ? q[j][i] : make_ulonglong2(0ull, 0ull);
+                const ulonglong2 at = pieces.at[k + 2u * r];
+                const uint64_t e = at.y + 2u * sub;
+                st_unit(at.x + 16u * sub, e, e + 1u, odd, pieces.units[k + 2u * r]);
             }
         }
-#pragma unroll
-        for(uint32_t j = 0; j < kPatternGroup; ++j)
+        __syncwarp();
+#pragma unroll 1
+        for(uint32_t k = half; k < total; k += 2u * kPatternRows)
         {
+            ulonglong2 v[kPatternRows];
 #pragma unroll
-            for(uint32_t u = 0; u < 2u; ++u)
+            for(uint32_t r = 0; r < kPatternRows; ++r)
+                v[r] = ld_unit(pieces.at[k + 2u * r].x + 16u * sub, odd, pieces.units[k + 2u * r]);
+            uint64_t diff = 0ull;
+#pragma unroll
+            for(uint32_t r = 0; r < kPatternRows; ++r)
             {
-                const uint32_t i = lane + 32u * u;
-                if(i < n16[j])
+                const uint64_t e = pieces.at[k + 2u * r].y + 2u * sub;
+                const uint32_t w = pieces.units[k + 2u * r];
+                const uint64_t d = (v[r].x ^ e) | (v[r].y ^ (e + 1u));
+                diff |= odd < w ? d : 0ull;
+                const uint64_t c = v[r].x ^ v[r].y;
+                if((w & 1u) == 0u)
+                    csum += c;
+                else
+                    other += c;
+            }
+            if(diff != 0ull)
+            {
+#pragma unroll
+                for(uint32_t r = 0; r < kPatternRows; ++r)
                 {
-                    bad += (v[j][u].x != mk[j] + 2u * i) + (v[j][u].y != mk[j] + 2u * i + 1u);
-                    csum += v[j][u].x ^ v[j][u].y;
+                    const uint64_t e = pieces.at[k + 2u * r].y + 2u * sub;
+                    if(odd < pieces.units[k + 2u * r])
+                        bad += (v[r].x != e) + (v[r].y != e + 1u);
                 }
             }
-            /* blocks above 1 KiB: the rest one 512-byte row at a time */
-            for(uint32_t i = lane + 64u; i < n16[j]; i += 32u)
-            {
-                const ulonglong2 w = q[j][i];
-                bad += (w.x != mk[j] + 2u * i) + (w.y != mk[j] + 2u * i + 1u);
-                csum += w.x ^ w.y;
-            }
         }
+        __syncwarp();
     }
-    __syncwarp();
     return bad;
 }
 
@@ -153,7 +182,8 @@ __global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h,
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nsizes = (p.hi - p.lo) / p.step + 1u;
     uint32_t pairs = 0, nulls = 0, bad = 0;
-    unsigned long long csum = 0;
+    unsigned long long csum = 0, other = 0;
+    __shared__ PatternPieces pieces[PATTERN == MMC_PATTERN_WARP ? 8 : 1]; /* a warp's each */
     for(uint32_t r = 0; r < p.rounds; ++r)
     {
         const uint64_t m = mix64(p.seed, t, r);
@@ -163,7 +193,7 @@ __global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h,
         if constexpr(PATTERN == MMC_PATTERN_WARP)
         {
             /* every lane takes part, with or without a block */
-            bad += warp_pattern(ptr, bytes, m, csum);
+            bad += warp_pattern(ptr, bytes, m, csum, other, pieces[threadIdx.x / 32u]);
             if(ptr == nullptr)
                 ++nulls;
             else
@@ -181,21 +211,13 @@ __global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h,
         }
         if constexpr(PATTERN == MMC_PATTERN_THREAD)
         {
-            /* 16-byte stores: chunks are 16-byte aligned under Shrink<16> */
-            ulonglong2* q = reinterpret_cast<ulonglong2*>(ptr);
-            const uint32_t n16 = bytes / 16u;
-            for(uint32_t i = 0; i < n16; ++i)
-                q[i] = make_ulonglong2(m + 2u * i, m + 2u * i + 1u);
-            for(uint32_t i = 0; i < n16; ++i)
-            {
-                const ulonglong2 v = q[i];
-                bad += (v.x != m + 2u * i) + (v.y != m + 2u * i + 1u);
-                csum += v.x ^ v.y;
-            }
+            thread_pattern<2>(ptr, bytes, m, bad, csum);
         }
         dv::free<Ids>(h, ptr);
         ++pairs;
     }
+    if constexpr(PATTERN == MMC_PATTERN_WARP)
+        csum += __shfl_xor_sync(0xFFFFFFFFu, other, 16);
     /* warp-aggregate the counters */
     for(int off = 16; off > 0; off >>= 1)
     {
@@ -222,7 +244,8 @@ __global__ void __launch_bounds__(256) mmc_stress_oldmalloc_kernel(mmc_stress_pa
     const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint32_t nsizes = (p.hi - p.lo) / p.step + 1u;
-    unsigned long long pairs = 0, nulls = 0, bad = 0, csum = 0;
+    unsigned long long pairs = 0, nulls = 0, bad = 0, csum = 0, other = 0;
+    __shared__ PatternPieces pieces[8]; /* a warp's each */
     for(uint32_t r = 0; r < p.rounds; ++r)
     {
         const uint64_t m = mix64(p.seed, t, r);
@@ -231,7 +254,7 @@ __global__ void __launch_bounds__(256) mmc_stress_oldmalloc_kernel(mmc_stress_pa
         char* ptr = static_cast<char*>(::malloc(bytes));
         if(p.write_pattern == MMC_PATTERN_WARP)
         {
-            bad += warp_pattern(ptr, bytes, m, csum);
+            bad += warp_pattern(ptr, bytes, m, csum, other, pieces[threadIdx.x / 32u]);
             if(ptr == nullptr)
                 ++nulls;
             else
@@ -252,21 +275,16 @@ __global__ void __launch_bounds__(256) mmc_stress_oldmalloc_kernel(mmc_stress_pa
         }
         if(p.write_pattern == MMC_PATTERN_THREAD)
         {
-            ulonglong2* q = reinterpret_cast<ulonglong2*>(ptr);
-            const uint32_t n16 = bytes / 16u;
-            for(uint32_t i = 0; i < n16; ++i)
-                q[i] = make_ulonglong2(m + 2u * i, m + 2u * i + 1u);
-            for(uint32_t i = 0; i < n16; ++i)
-            {
-                const ulonglong2 v = q[i];
-                bad += (v.x != m + 2u * i) + (v.y != m + 2u * i + 1u);
-                csum += v.x ^ v.y;
-            }
+            uint32_t wrong = 0;
+            thread_pattern<2>(ptr, bytes, m, wrong, csum);
+            bad += wrong;
         }
         dv::release_fence();
         ::free(ptr);
         ++pairs;
     }
+    if(p.write_pattern == MMC_PATTERN_WARP)
+        csum += __shfl_xor_sync(0xFFFFFFFFu, other, 16);
     for(int off = 16; off > 0; off >>= 1)
     {
         pairs += __shfl_down_sync(0xFFFFFFFFu, pairs, off);
