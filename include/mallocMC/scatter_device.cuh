@@ -278,40 +278,10 @@ namespace mmc
             const u32 high_part = (bitfield << (spots - (spot + 1u)));
             const u32 selection_mask = spots == 32u ? ~0u : ((1u << spots) - 1u);
             bitfield = (high_part | low_part) & selection_mask;
-            const u32 step = static_cast<u32>(__ffs(static_cast<int>(~bitfield)));
-            return (spot + step) % spots;
-        }
-
-        /* usespot's retry sequence (Scatter.hpp:334-346) after an atomicOr at
-         * `spot` returned `old` with that bit already set: stop when the word is
-         * full, else try the next free spot of the returned word. Bounded by
-         * MMC_USESPOT_MAX_TRIES lost races, after which the word counts as full,
-         * which every caller already handles. */
-        __device__ __forceinline__ int usespot_continue(u32* bitfield, u32 spots, u32 spot, u32 old)
-        {
-            for(u32 it = 1; it < MMC_USESPOT_MAX_TRIES; ++it)
-            {
-                if(static_cast<u32>(__popc(old)) >= spots)
-                    return -1;
-                spot = nextspot(old, spot, spots);
-                const u32 mask = 1u << spot;
-                old = atomicOr(bitfield, mask);
-                if((old & mask) == 0u)
-                    return static_cast<int>(spot);
-            }
-            return -1;
-        }
-
-        /* usespot, Scatter.hpp:329-347 (first spot laneid % spots, randInit :277-281) */
-        template<class Ids>
-        __device__ __forceinline__ int usespot(u32* bitfield, u32 spots)
-        {
-            const u32 spot = Ids::laneid() % spots;
-            const u32 mask = 1u << spot;
-            const u32 old = atomicOr(bitfield, mask);
-            if((old & mask) == 0u)
-                return static_cast<int>(spot);
-            return usespot_continue(bitfield, spots, spot, old);
+            /* (spot + step) % spots; step is at most spots + 1 */
+            u32 next = spot + static_cast<u32>(__ffs(static_cast<int>(~bitfield)));
+            next -= next >= spots ? spots : 0u;
+            return next - (next >= spots ? spots : 0u);
         }
 
         /* calcAdditionalChunks, Scatter.hpp:365-381: the (int) casts collapse to
@@ -363,64 +333,68 @@ namespace mmc
 
         /* Claim one chunk on a page whose fill slot is reserved:
          * addChunkHierarchy (Scatter.hpp:397-421) for hierarchical pages,
-         * addChunkNoHierarchy (:432-443) otherwise. Both begin with one atomicOr
-         * on a per-lane word (a segment's on-page mask or the page bitmask), so
-         * the lanes of a warp issue that first claim as a single instruction
-         * whatever their page kind; a lane that loses the race continues the
-         * reference's exact retry sequence. `mask` is the page's segment hints. */
+         * addChunkNoHierarchy (:432-443) otherwise, both over usespot
+         * (:329-347, first spot laneid % spots, randInit :277-281): atomicOr a
+         * bit of a word (a segment's on-page mask or the page bitmask); when it
+         * was set already, stop if the word is full, else try the next free
+         * spot of the returned word. MMC_USESPOT_MAX_TRIES lost races count as
+         * a full word, which every caller handles. `mask` is the page's
+         * segment hints. One loop with one atomicOr serves both page kinds and
+         * every retry: the copies of an unrolled retry loop in front of each
+         * of them were most of a kernel's code (see alloc_chunked). */
         template<class Ids>
-        __device__ void* claim_chunk(const mmc_device_handle& h, u32 page, u32 chunksize, const ChunkGeom& g, u32 mask)
+        __device__ __forceinline__ void* claim_chunk(const mmc_device_handle& h, u32 page, u32 chunksize,
+                                                     const ChunkGeom& g, u32 mask)
         {
-            u32* word;
-            u32 spots;
+            u32* word = &h.bitmask[page];
+            u32 spots = g.capacity;
             u32 seg = 0u;
             u32 tries = 1u;
-            u32* onpagemasks = nullptr;
             if(g.hier)
             {
                 seg = Ids::laneid() % g.segments;
                 if((mask & (1u << seg)) != 0u)
                     seg = nextspot(mask, seg, g.segments);
                 tries = g.segments - static_cast<u32>(__popc(mask));
-                onpagemasks = on_page_masks(h, page, g.segments);
-                word = onpagemasks + seg;
+                word = on_page_masks(h, page, g.segments) + seg;
                 spots = seg < g.fullsegments ? 32u : g.additional;
             }
-            else
+            u32 spot = Ids::laneid() % spots;
+            u32 races = 0u;
+            bool claimed = false;
+#pragma unroll 1
+            while(!claimed && tries != 0u)
             {
-                word = &h.bitmask[page];
-                spots = g.capacity;
+                const u32 bit = 1u << spot;
+                const u32 old = atomicOr(word, bit);
+                claimed = (old & bit) == 0u;
+                if(!claimed)
+                {
+                    if(static_cast<u32>(__popc(old)) < spots && ++races < MMC_USESPOT_MAX_TRIES)
+                        spot = nextspot(old, spot, spots);
+                    else if(--tries != 0u || g.hier)
+                    {
+                        atomicOr(&h.bitmask[page], 1u << seg);
+                        /* A free in this segment may have cleared the hint just before
+                         * it was set; undo a mark the segment no longer deserves so no
+                         * stale "full" bit outlives the chunks. A lone thread only gets
+                         * here for a full segment, so this never fires serially. */
+                        if(static_cast<u32>(__popc(ld_rlx(word))) < spots)
+                            atomicAnd(&h.bitmask[page], ~(1u << seg));
+                        seg = nextspot(mask, seg, g.segments);
+                        word = on_page_masks(h, page, g.segments) + seg;
+                        spots = seg < g.fullsegments ? 32u : g.additional;
+                        spot = Ids::laneid() % spots;
+                        races = 0u;
+                    }
+                }
             }
-            if(tries == 0u)
-                return nullptr;
-            const u32 spot = Ids::laneid() % spots;
-            const u32 bit = 1u << spot;
-            const u32 old = atomicOr(word, bit);
-            int got = (old & bit) == 0u ? static_cast<int>(spot) : usespot_continue(word, spots, spot, old);
-            if(!g.hier)
-                return got == -1 ? nullptr : page_data(h, page) + static_cast<u32>(got) * chunksize;
-            for(u32 i = 0;;)
-            {
-                if(got != -1)
-                    return page_data(h, page) + (32u * seg + static_cast<u32>(got)) * chunksize;
-                atomicOr(&h.bitmask[page], 1u << seg);
-                /* A free in this segment may have cleared the hint just before
-                 * it was set; undo a mark the segment no longer deserves so no
-                 * stale "full" bit outlives the chunks. A lone thread only gets
-                 * here for a full segment, so this never fires serially. */
-                if(static_cast<u32>(__popc(ld_rlx(&onpagemasks[seg]))) < spots)
-                    atomicAnd(&h.bitmask[page], ~(1u << seg));
-                seg = nextspot(mask, seg, g.segments);
-                if(++i >= tries)
-                    return nullptr;
-                spots = seg < g.fullsegments ? 32u : g.additional;
-                got = usespot<Ids>(&onpagemasks[seg], spots);
-            }
+            return claimed ? page_data(h, page) + (32u * seg + spot) * chunksize : nullptr;
         }
 
         /* tryUsePage, Scatter.hpp:454-518; [lo, hi] is isChunkSizeInRange (:586-588). */
         template<class Ids>
-        __device__ void* try_use_page(const mmc_device_handle& h, u32 page, u32 chunksize, u32 lo, u32 hi)
+        __device__ __forceinline__ void* try_use_page(const mmc_device_handle& h, u32 page, u32 chunksize, u32 lo, u32 hi)
         {
             void* chunk_ptr = nullptr;
             /* the segment hints are read before the fill-count atomic so both
@@ -521,120 +495,148 @@ namespace mmc
             }
         }
 
-        /* allocChunked's two-pass region walk (Scatter.hpp:563-636), resumed after
-         * the first page: in the first region of pass 0 the region counter is
-         * the one already read (fill0) and the start page was already tried.
+        /* allocChunked's two-pass region walk (Scatter.hpp:563-636), resumed
+         * after the start page: in the first region of pass 0 the region
+         * counter is the one already read (level) and the start page was tried.
+         * Every region is read whole (region_candidates: one round trip for 16
+         * pages) and only its usable pages are tried, in the reference's order
+         * from the entry page: a walk that crosses regions of full pages or of
+         * multi-page runs (the page-based area, where region counters stay low
+         * because only failed chunk walks raise them) costs one round trip per
+         * region instead of one per page. The region counters are looked at
+         * eight regions ahead, so a stretch of regions skipped as 3/4 full
+         * costs one round trip per eight. Alone on the heap every page gets
+         * the reference's outcome, in the reference's order.
          *
-         * That first region is walked page by page, as the reference walks it
-         * (most walks end there, after a page or two). Every further region is
-         * read whole first (region_candidates: one round trip for 16 pages) and
-         * only its usable pages are tried, in the reference's order from the
-         * entry page: a walk that crosses regions of full pages or of multi-page
-         * runs (the page-based area, where region counters stay low because
-         * only failed chunk walks raise them) then costs one round trip per
-         * region instead of one per page. The region counters themselves are
-         * read eight regions ahead, so a stretch of regions skipped as 3/4 full
-         * costs one round trip per eight (a walk only changes the counter of the
-         * region it is in). Alone on the heap every page gets the reference's
-         * outcome, in the reference's order. */
+         * The warp's walking lanes go step by step together: per step each
+         * moves to its next region if it has to and tries one page. Left to
+         * itself the compiler threads the jumps of the lanes that pass a page
+         * around those that try one, and they no longer meet (up to twice the
+         * instructions on the uniform stress). One attempt serves every page,
+         * and malloc has one call of all this: with an attempt for each kind
+         * of region, each with unrolled claim retries, and two call sites in
+         * malloc, a kernel that allocates had 100 to 180 KB of code, and
+         * instruction fetch was the first stall of the stress and batched
+         * kernels. */
         template<class Ids>
-        __device__ void* alloc_chunked_walk(const mmc_device_handle& h, u32 bytes, u32 minAllocation,
-                                            u32 maxchunksize, u32 global_start_page, u32 fill0)
+        __device__ __forceinline__ void* alloc_chunked_walk(const mmc_device_handle& h, u32 bytes, u32 minAllocation,
+                                                            u32 maxchunksize, u32 start, u32 level)
         {
             const u32 R = h.regionsize;
-            const u32 numpages = h.numpages;
             const u32 numregions = h.numregions;
-            const u32 pagesperblock = h.pagesperblock;
             const bool batched = (R % 4u) == 0u && R <= 32u;
             const u32 rmask = R >= 32u ? 0xFFFFFFFFu : ((1u << R) - 1u);
-            constexpr u32 kAhead = 8u;
+            u32 region = start / R;
+            const u32 s0 = start - region * R;
             u32 checklevel = R * 3u / 4u;
-            for(u32 finder = 0; finder < 2u; ++finder)
+            u64 ahead = 0u; /* counters of the regions ahead, a byte each */
+            u32 known = 1u; /* how many, with this one */
+            u32 left = 2u * numregions; /* regions to visit, in both passes, this one included */
+            /* Visiting index i is page region * R + (s0 + i) % R. With masks, the
+             * usable pages (todo) and the unformatted ones (zero) go by it;
+             * without, i is the last page visited. */
+            u32 todo = 0u, zero = 0u, i = 0u;
+            bool masks = false;
+            bool walking = level < checklevel;
+            if(!walking)
+                i = R;
+            void* res = nullptr;
+            bool go = true;
+            u32 am = 1u;
+            if constexpr(Ids::warpSize > 1u)
+                am = __activemask();
+            do
             {
-                u32 global_page = global_start_page;
-                u32 ahead[kAhead];
-                u32 ahead_left = 0u; /* counters of the next regions already read */
-                do
+                if(go && (masks ? todo == 0u : i + 1u >= R))
                 {
-                    const u32 region = global_page / R;
-                    const bool resumed = finder == 0u && global_page == global_start_page;
-                    if(!resumed && ahead_left == 0u)
+                    /* the region has no page left to try: on to the next one to walk */
+                    if(walking)
                     {
-#pragma unroll
-                        for(u32 k = 0; k < kAhead; ++k)
-                        {
-                            u32 r = region + k;
-                            r = r >= numregions ? r - numregions : r;
-                            ahead[k] = ld_rlx(&h.regions[r]);
-                        }
-                        ahead_left = kAhead;
-                    }
-                    u32 regionfilllevel = fill0;
-                    if(!resumed)
-                    {
-                        regionfilllevel = ahead[kAhead - ahead_left];
-                        --ahead_left;
-                    }
-                    const u32 region_offset = region * R;
-                    if(regionfilllevel < checklevel)
-                    {
-                        if(batched && !resumed)
-                        {
-                            u32 zero, fit;
-                            region_candidates(h, region_offset, bytes, maxchunksize, zero, fit);
-                            /* rotate so that bit i is the i-th page visited from the entry page */
-                            const u32 s0 = global_page - region_offset;
-                            const u32 z = s0 == 0u ? zero : (((zero >> s0) | (zero << (R - s0))) & rmask);
-                            const u32 f = s0 == 0u ? fit : (((fit >> s0) | (fit << (R - s0))) & rmask);
-                            for(u32 todo = z | f; todo != 0u; todo &= todo - 1u)
-                            {
-                                const u32 i = static_cast<u32>(__ffs(static_cast<int>(todo))) - 1u;
-                                const u32 page = region_offset + (s0 + i) % R;
-                                MMC_STAT(h, MMC_STAT_WALK_PAGES);
-                                const u32 before = ((z >> i) & 1u) ? 0u : ld_rlx(&h.chunksize[page]);
-                                void* res = attempt_page<Ids>(h, page, before, bytes, minAllocation, maxchunksize);
-                                if(res != nullptr)
-                                    return res;
-                            }
-                        }
-                        else
-                        {
-                            u32 page_in_region = global_page;
-                            bool skip = resumed;
-                            do
-                            {
-                                if(!skip)
-                                {
-                                    MMC_STAT(h, MMC_STAT_WALK_PAGES);
-                                    void* res = attempt_page<Ids>(h, page_in_region,
-                                                                  ld_rlx(&h.chunksize[page_in_region]), bytes,
-                                                                  minAllocation, maxchunksize);
-                                    if(res != nullptr)
-                                        return res;
-                                }
-                                skip = false;
-                                page_in_region = region_offset + ((page_in_region + 1u) % R);
-                            } while(page_in_region != global_page);
-                        }
-
-                        if(regionfilllevel + 1u <= R)
-                            atomicCAS(&h.regions[region], regionfilllevel, regionfilllevel + 1u);
+                        if(level == 255u)
+                            level = ld_rlx(&h.regions[region]);
+                        if(level + 1u <= R)
+                            atomicCAS(&h.regions[region], level, level + 1u);
                         MMC_STAT(h, MMC_STAT_REGION_FAIL);
                     }
                     else
                         MMC_STAT(h, MMC_STAT_REGION_SKIP);
-                    global_page = (global_page + R) % numpages;
-                    if(global_page % pagesperblock == 0u)
+                    if(++region == numregions)
+                        region = 0u;
+                    if(s0 == 0u && (region * R) % h.pagesperblock == 0u)
                     {
-                        const u32 access_block_id = global_page / pagesperblock;
+                        const u32 access_block_id = region * R / h.pagesperblock;
                         /* racy by design (Scatter.hpp:625-628) */
                         if(access_block_id > ld_rlx(&h.state->firstfreeblock))
                             st_rlx(&h.state->firstfreeblock, access_block_id);
                     }
-                } while(global_page != global_start_page);
-                checklevel = R + 1u;
-            }
-            return nullptr;
+                    ahead >>= 8;
+                    --known;
+                    if(--left == numregions)
+                    {
+                        /* the second pass walks every region */
+                        checklevel = R + 1u;
+                        known = 0u;
+                    }
+                    go = left != 0u;
+                    if(known == 0u && go)
+                    {
+                        known = umin(8u, numregions - region);
+                        ahead = 0u;
+#pragma unroll
+                        for(u32 k = 0; k < 8u; ++k)
+                            if(k < known)
+                                ahead |= static_cast<u64>(umin(ld_rlx(&h.regions[region + k]), 255u)) << (8u * k);
+                    }
+                    /* The counter as it was looked at, up to eight regions
+                     * ago: of several walks that fail here together one
+                     * raises it, not each. (With a fresh look it rises with
+                     * every failed walk; regions with free chunks are then
+                     * passed sooner, and the refill of the 32 GiB
+                     * fragmentation run formatted 440 to 480 thousand pages
+                     * for chunks instead of 427.) */
+                    level = static_cast<u32>(ahead) & 255u;
+                    walking = go && level < checklevel;
+                    masks = batched;
+                    todo = 0u;
+                    i = walking ? ~0u : R;
+                    if(walking)
+                    {
+                        if(masks)
+                        {
+                            region_candidates(h, region * R, bytes, maxchunksize, zero, todo);
+                            if(s0 != 0u)
+                            {
+                                zero = ((zero >> s0) | (zero << (R - s0))) & rmask;
+                                todo = ((todo >> s0) | (todo << (R - s0))) & rmask;
+                            }
+                            todo |= zero;
+                        }
+                    }
+                }
+                if(go && (masks ? todo != 0u : i + 1u < R))
+                {
+                    ++i;
+                    if(masks)
+                    {
+                        i = static_cast<u32>(__ffs(static_cast<int>(todo))) - 1u;
+                        todo &= todo - 1u;
+                    }
+                    const u32 off = s0 + i;
+                    const u32 page = region * R + (off >= R ? off - R : off);
+                    MMC_STAT(h, MMC_STAT_WALK_PAGES);
+                    const u32 before = masks && ((zero >> i) & 1u) != 0u ? 0u : ld_rlx(&h.chunksize[page]);
+                    res = attempt_page<Ids>(h, page, before, bytes, minAllocation, maxchunksize);
+                    go = res == nullptr;
+                }
+                if constexpr(Ids::warpSize > 1u)
+                {
+                    if(!__any_sync(am, go))
+                        break;
+                }
+                else if(!go)
+                    break;
+            } while(true);
+            return res;
         }
 
         /* One page of a same-size group claim, by the group's leader: reserve up
@@ -653,12 +655,14 @@ namespace mmc
             const u32 full = cap == 32u ? 0xFFFFFFFFu : ((1u << cap) - 1u);
             u32 mask = grant != 0u ? ld_rlx(&h.bitmask[page]) : full;
             u32 got = 0u;
+#pragma unroll 1
             for(u32 tries = 0; grant != 0u && tries < MMC_USESPOT_MAX_TRIES; ++tries)
             {
                 u32 free = ~mask & full;
                 if(free == 0u)
                     break;
                 u32 pick = 0u;
+#pragma unroll 1
                 for(u32 n = 0; n < grant && free != 0u; ++n)
                 {
                     pick |= free & (0u - free); /* lowest free bit */
@@ -713,6 +717,7 @@ namespace mmc
                 return false;
             u32 served = 0u;
             u32 page = start;
+#pragma unroll 1
             for(u32 visited = 0; visited < R && served < k; ++visited)
             {
                 u32 got = 0u, use = 0u;
@@ -734,6 +739,7 @@ namespace mmc
                 if(rank >= served && rank < served + n)
                 {
                     u32 m = got;
+#pragma unroll 1
                     for(u32 i = served; i < rank; ++i)
                         m &= m - 1u;
                     const u32 bit = static_cast<u32>(__ffs(static_cast<int>(m))) - 1u;
@@ -755,7 +761,7 @@ namespace mmc
          * code every lane of a warp executes in step; only lanes whose first
          * page fails enter the (divergent) rest of the walk. */
         template<class Ids>
-        __device__ void* alloc_chunked(const mmc_device_handle& h, u32 bytes)
+        __device__ __forceinline__ void* alloc_chunked(const mmc_device_handle& h, u32 bytes)
         {
             const u32 P = h.pagesize;
             const u32 R = h.regionsize;
@@ -775,24 +781,26 @@ namespace mmc
             const u32 fill0 = ld_rlx(&h.regions[global_start_page / R]);
             const u32 cs0 = ld_rlx(&h.chunksize[global_start_page]);
             MMC_STAT(h, MMC_STAT_CHUNKED);
+            void* res = nullptr;
+            bool served = false;
             if constexpr(Ids::warpSize > 1u)
             {
-                void* grouped = nullptr;
-                if(claim_same_size<Ids>(h, bytes, minAllocation, maxchunksize, global_start_page, fill0, cs0, grouped))
-                    return grouped;
+                const u32 am = __activemask();
+                served = claim_same_size<Ids>(h, bytes, minAllocation, maxchunksize, global_start_page, fill0, cs0, res);
+                __syncwarp(am);
             }
-            if(fill0 < R * 3u / 4u)
+            if(!served && fill0 < R * 3u / 4u)
             {
-                void* res = attempt_page<Ids>(h, global_start_page, cs0, bytes, minAllocation, maxchunksize);
+                res = attempt_page<Ids>(h, global_start_page, cs0, bytes, minAllocation, maxchunksize);
                 if(res != nullptr)
-                {
                     MMC_STAT(h, MMC_STAT_FIRST_PAGE);
-                    return res;
-                }
             }
-            void* res = alloc_chunked_walk<Ids>(h, bytes, minAllocation, maxchunksize, global_start_page, fill0);
             if(res == nullptr)
-                MMC_STAT(h, MMC_STAT_CHUNKED_FAIL);
+            {
+                res = alloc_chunked_walk<Ids>(h, bytes, minAllocation, maxchunksize, global_start_page, fill0);
+                if(res == nullptr)
+                    MMC_STAT(h, MMC_STAT_CHUNKED_FAIL);
+            }
             return res;
         }
 
@@ -1406,75 +1414,87 @@ namespace mmc
         __device__ void* malloc(const mmc_device_handle& h, size_t bytes_in)
         {
             const u32 bytes = apply_padding(Ids::alignment(h), static_cast<u32>(bytes_in));
-            if(!Ids::coalesce || Ids::distribution(h) != MMC_DIST_XMALLOCSIMD)
-            {
-                void* p = create<Ids>(h, bytes);
-                return handle_oom<Ids>(h, p, bytes);
-            }
-            const u32 active = __activemask();
-            const bool coalescible = bytes > 0u && bytes < (h.pagesize / 32u);
-            const u32 cmask = __ballot_sync(active, coalescible);
-            const u32 threadcount = static_cast<u32>(__popc(cmask));
-            if(threadcount <= 1u)
-            {
-                void* p = create<Ids>(h, bytes);
-                return handle_oom<Ids>(h, p, bytes);
-            }
-            /* exclusive prefix of the coalescible lanes' sizes, in lane order */
-            const u32 lane = Ids::laneid();
-            const u32 mine = coalescible ? bytes : 0u;
-            u32 before = 0u;
-            if(active == 0xFFFFFFFFu)
-            {
-                u32 incl = mine;
-#pragma unroll
-                for(u32 off = 1u; off < 32u; off <<= 1)
-                {
-                    const u32 v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-                    if(lane >= off)
-                        incl += v;
-                }
-                before = incl - mine;
-            }
-            else
-            {
-                for(u32 m = cmask; m != 0u; m &= m - 1u)
-                {
-                    const u32 src = static_cast<u32>(__ffs(static_cast<int>(m))) - 1u;
-                    const u32 v = __shfl_sync(active, mine, static_cast<int>(src));
-                    if(src < lane)
-                        before += v;
-                }
-            }
-            const u32 total = __reduce_add_sync(active, mine);
-            const u32 leader = static_cast<u32>(__ffs(static_cast<int>(cmask))) - 1u;
+            /* one call of create for every form, so its code is in the kernel once */
             u32 req = bytes;
-            if(coalescible)
-                req = (lane == leader) ? 16u + total : 0u;
+            u32 active = 1u, threadcount = 0u, before = 0u, leader = 0u;
+            bool coalescible = false;
+            if constexpr(Ids::warpSize > 1u)
+                active = __activemask();
+            const u32 lane = Ids::laneid();
+            if(Ids::coalesce && Ids::distribution(h) == MMC_DIST_XMALLOCSIMD)
+            {
+                coalescible = bytes > 0u && bytes < (h.pagesize / 32u);
+                const u32 cmask = __ballot_sync(active, coalescible);
+                threadcount = static_cast<u32>(__popc(cmask));
+                if(threadcount > 1u)
+                {
+                    /* exclusive prefix of the coalescible lanes' sizes, in lane order */
+                    const u32 mine = coalescible ? bytes : 0u;
+                    if(active == 0xFFFFFFFFu)
+                    {
+                        u32 incl = mine;
+#pragma unroll
+                        for(u32 off = 1u; off < 32u; off <<= 1)
+                        {
+                            const u32 v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+                            if(lane >= off)
+                                incl += v;
+                        }
+                        before = incl - mine;
+                    }
+                    else
+                    {
+#pragma unroll 1
+                        for(u32 m = cmask; m != 0u; m &= m - 1u)
+                        {
+                            const u32 src = static_cast<u32>(__ffs(static_cast<int>(m))) - 1u;
+                            const u32 v = __shfl_sync(active, mine, static_cast<int>(src));
+                            if(src < lane)
+                                before += v;
+                        }
+                    }
+                    const u32 total = __reduce_add_sync(active, mine);
+                    leader = static_cast<u32>(__ffs(static_cast<int>(cmask))) - 1u;
+                    if(coalescible)
+                        req = (lane == leader) ? 16u + total : 0u;
+                }
+                else
+                    coalescible = false;
+            }
+            /* the leader and the lanes on their own search together */
+            if constexpr(Ids::warpSize > 1u)
+                __syncwarp(active);
             void* mem = create<Ids>(h, req);
             mem = handle_oom<Ids>(h, mem, req);
-            if(coalescible && lane == leader && mem != nullptr)
+            if constexpr(Ids::warpSize > 1u)
             {
-                st_rlx(static_cast<u32*>(mem), threadcount);
-                /* The count's sector is usually cold, and the store leaves it
-                 * partly valid in L2: the frees' atomics on it would wait for
-                 * the DRAM fill. Fetch it now, while the lanes use their parts. */
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(mem));
+                if(coalescible && lane == leader && mem != nullptr)
+                {
+                    st_rlx(static_cast<u32*>(mem), threadcount);
+                    /* The count's sector is usually cold, and the store leaves it
+                     * partly valid in L2: the frees' atomics on it would wait for
+                     * the DRAM fill. Fetch it now, while the lanes use their parts. */
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(mem));
+                }
+                /* The lane count must be seen by every later free of a sub-allocation
+                 * (device-scope atomicSubs on this word). The warp barrier orders
+                 * the leader's store before every lane's accesses after it, the
+                 * frees included; a free by another thread is ordered through the
+                 * synchronisation that handed it the pointer. (The reference stores
+                 * the count with a block-scope fence, XMallocSIMD.hpp:160-166; a
+                 * device-scope fence here measured 3-5 % slower on the batched
+                 * workload.) It also brings the lanes together again after their
+                 * searches. */
+                __syncwarp(active);
+                if(threadcount > 1u)
+                {
+                    const unsigned long long base
+                        = __shfl_sync(active, reinterpret_cast<unsigned long long>(mem), static_cast<int>(leader));
+                    if(coalescible)
+                        mem = base != 0ull ? reinterpret_cast<char*>(base) + 16u + before : nullptr;
+                }
             }
-            /* The lane count must be seen by every later free of a sub-allocation
-             * (device-scope atomicSubs on this word). The warp barrier orders
-             * the leader's store before every lane's accesses after it, the
-             * frees included; a free by another thread is ordered through the
-             * synchronisation that handed it the pointer. (The reference stores
-             * the count with a block-scope fence, XMallocSIMD.hpp:160-166; a
-             * device-scope fence here measured 3-5 % slower on the batched
-             * workload.) */
-            __syncwarp(active);
-            const unsigned long long base
-                = __shfl_sync(active, reinterpret_cast<unsigned long long>(mem), static_cast<int>(leader));
-            if(!coalescible)
-                return mem;
-            return base != 0ull ? reinterpret_cast<char*>(base) + 16u + before : nullptr;
+            return mem;
         }
 
         template<class Ids>
