@@ -51,6 +51,21 @@ struct mmc_heap_state
     unsigned long long stats[16];
 };
 
+/* Multi-page requests of whole warps waiting to be served (see
+ * page_service_run): a ring of tickets. It follows mmc_heap_state in the
+ * heap's device block. */
+#define MMC_PAGE_RING 32768u
+struct mmc_page_service
+{
+    uint32_t lock; /* held by the warp that serves */
+    uint32_t pad0[31];
+    uint32_t tail; /* tickets handed out */
+    uint32_t pad1[31];
+    uint32_t head; /* tickets served; the lock's holder moves it */
+    uint32_t pad2[31];
+    uint32_t ring[MMC_PAGE_RING]; /* 0: idle; kPageAsk | pages: waiting; else the answer */
+};
+
 #ifdef MMC_DEVICE_STATS
 #define MMC_STAT(h, i) atomicAdd(&(h).state->stats[(i)], 1ull)
 #define MMC_STAT_ADD(h, i, n) atomicAdd(&(h).state->stats[(i)], static_cast<unsigned long long>(n))
@@ -192,6 +207,10 @@ namespace mmc
             asm("mov.u32 %0, %%lanemask_lt;" : "=r"(r));
             return r;
         }
+        /* The lanes that run here together, as a value to keep: a bare
+         * activemask may be read again by the compiler where the lanes have
+         * parted, and barriers on what it then gives wait for one another. */
+        __device__ __forceinline__ u32 converged_lanes() { return __ballot_sync(__activemask(), true); }
         __device__ __forceinline__ u32 umin(u32 a, u32 b) { return a < b ? a : b; }
         __device__ __forceinline__ u32 umax(u32 a, u32 b) { return a > b ? a : b; }
         __device__ __forceinline__ u32 divup(u32 a, u32 b) { return (a + b - 1u) / b; }
@@ -459,17 +478,28 @@ namespace mmc
 
         /* The pages of one region a request may use, as two masks in page order
          * (bit i = page region_offset + i): unformatted pages (chunk size 0) and
-         * pages formatted with a chunk size in [bytes, maxchunksize]. Every other
-         * page is one the reference's walk visits only to find it formatted for
-         * another size or taken by a multi-page run (Scatter.hpp:584-591). The
-         * chunk-size words are read with 16-byte loads, 16 pages in flight at
-         * once. Needs regionsize % 4 == 0 and regionsize <= 32. */
+         * pages formatted with a chunk size in [bytes, maxchunksize] that have
+         * a chunk free. Every other page is one the reference's walk visits
+         * only to find it formatted for another size, taken by a multi-page run
+         * (Scatter.hpp:584-591) or full (:500). Chunk sizes, and where there
+         * are chunk pages their fill counts, are read with 16-byte loads, 16 or
+         * eight pages at once: a walk costs one round trip per region of
+         * multi-page runs and three per region of full chunk pages, where
+         * reserving a fill slot on each page and giving it back cost two per
+         * page. (Keeping the chunk sizes of 16 pages for the second step takes
+         * one round trip less and spilled 370 bytes of the stress kernel.) Pages of
+         * chunks up to HierarchyThreshold (whose capacity takes two divisions)
+         * are left to the attempt. `room`: the region has a page or a chunk of
+         * any size free. Needs regionsize % 4 == 0 and regionsize <= 32. */
         __device__ __forceinline__ void region_candidates(const mmc_device_handle& h, u32 region_offset, u32 bytes,
-                                                          u32 maxchunksize, u32& zero, u32& fit)
+                                                          u32 maxchunksize, u32& zero, u32& fit, bool& room)
         {
             const u32 R = h.regionsize;
             zero = 0u;
             fit = 0u;
+            room = false;
+            u32 chunks = 0u; /* pages formatted for chunks */
+#pragma unroll 1
             for(u32 base = 0; base < R; base += 16u)
             {
                 uint4 v[4];
@@ -484,29 +514,67 @@ namespace mmc
 #pragma unroll
                     for(u32 j = 0; j < 4u; ++j)
                     {
-                        const u32 bit = base + 4u * k + j;
-                        if(bit < 32u)
-                        {
-                            zero |= (w[j] == 0u ? 1u : 0u) << bit;
-                            fit |= ((w[j] >= bytes && w[j] <= maxchunksize) ? 1u : 0u) << bit;
-                        }
+                        zero |= (w[j] == 0u ? 1u : 0u) << ((base + 4u * k + j) & 31u);
+                        chunks |= (w[j] - 1u < h.pagesize ? 1u : 0u) << ((base + 4u * k + j) & 31u);
                     }
                 }
             }
+#pragma unroll 1
+            for(u32 base = 0; chunks >> base != 0u; base += 8u)
+            {
+                uint4 v[2], c[2];
+#pragma unroll
+                for(u32 k = 0; k < 2u; ++k)
+                {
+                    const bool in = base + 4u * k < R;
+                    v[k] = in ? ld_rlx_v4(&h.chunksize[region_offset + base + 4u * k]) : make_uint4(~0u, ~0u, ~0u, ~0u);
+                    c[k] = in ? ld_rlx_v4(&h.count[region_offset + base + 4u * k]) : make_uint4(0u, 0u, 0u, 0u);
+                }
+#pragma unroll
+                for(u32 k = 0; k < 2u; ++k)
+                {
+                    const u32 w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+                    const u32 n[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
+#pragma unroll
+                    for(u32 j = 0; j < 4u; ++j)
+                    {
+                        const bool more = n[j] < 32u * 33u && (n[j] + 1u) * w[j] <= h.pagesize;
+                        fit |= (w[j] >= bytes && w[j] <= maxchunksize && (more || w[j] <= h.hierarchyThreshold) ? 1u : 0u)
+                            << (base + 4u * k + j);
+                        room = room || more;
+                    }
+                }
+                if(base == 24u)
+                    break;
+            }
+            room = room || zero != 0u;
         }
 
         /* allocChunked's two-pass region walk (Scatter.hpp:563-636), resumed
          * after the start page: in the first region of pass 0 the region
          * counter is the one already read (level) and the start page was tried.
-         * Every region is read whole (region_candidates: one round trip for 16
-         * pages) and only its usable pages are tried, in the reference's order
-         * from the entry page: a walk that crosses regions of full pages or of
-         * multi-page runs (the page-based area, where region counters stay low
-         * because only failed chunk walks raise them) costs one round trip per
-         * region instead of one per page. The region counters are looked at
+         * The rest of that region is walked page by page, as the reference
+         * walks it: most walks end there, after a page or two. Every further
+         * region is read whole (region_candidates) and only its usable pages
+         * are tried, in the reference's order from the entry page: a walk that
+         * crosses regions of full pages or of multi-page runs costs a few
+         * round trips per region instead of one or two per page. The region counters are looked at
          * eight regions ahead, so a stretch of regions skipped as 3/4 full
          * costs one round trip per eight. Alone on the heap every page gets
          * the reference's outcome, in the reference's order.
+         *
+         * The counters: the reference counts every failed walk, whatever size
+         * it wanted, and passes regions that 3/4 * R have failed in. Many
+         * threads raise them that far at once, in regions that still have room
+         * for other sizes; walks then pass whole blocks with free chunks, the
+         * first-free-block hint follows them, and new pages are formatted
+         * further on. For concurrent callers a walk counts only in a region
+         * with no page free and no chunk free of any size, and only in the
+         * first pass (the second walks every region anyway, and would mark the
+         * whole heap). The 32 GiB fragmentation run, whose multi-page requests
+         * are served fast enough to fill the heap to its last page: 0.9713 of
+         * the heap after its refill counting every walk, 0.9783 this way (the
+         * reference's serial run: 0.9750).
          *
          * The warp's walking lanes go step by step together: per step each
          * moves to its next region if it has to and tries one page. Left to
@@ -537,6 +605,7 @@ namespace mmc
              * without, i is the last page visited. */
             u32 todo = 0u, zero = 0u, i = 0u;
             bool masks = false;
+            bool room = true; /* the region has a page or a chunk of some size free */
             bool walking = level < checklevel;
             if(!walking)
                 i = R;
@@ -544,17 +613,20 @@ namespace mmc
             bool go = true;
             u32 am = 1u;
             if constexpr(Ids::warpSize > 1u)
-                am = __activemask();
+                am = converged_lanes();
             do
             {
-                if(go && (masks ? todo == 0u : i + 1u >= R))
+                bool read = false;
+                if(Ids::warpSize > 1u && go && walking && batched && !masks && i + 1u >= R)
+                    read = true; /* walked page by page: is it full? */
+                else if(go && (masks ? todo == 0u : i + 1u >= R))
                 {
                     /* the region has no page left to try: on to the next one to walk */
-                    if(walking)
+                    if(walking && (Ids::warpSize == 1u || !batched || !room))
                     {
                         if(level == 255u)
                             level = ld_rlx(&h.regions[region]);
-                        if(level + 1u <= R)
+                        if(level + 1u <= R && (Ids::warpSize == 1u || checklevel <= R))
                             atomicCAS(&h.regions[region], level, level + 1u);
                         MMC_STAT(h, MMC_STAT_REGION_FAIL);
                     }
@@ -587,31 +659,25 @@ namespace mmc
                             if(k < known)
                                 ahead |= static_cast<u64>(umin(ld_rlx(&h.regions[region + k]), 255u)) << (8u * k);
                     }
-                    /* The counter as it was looked at, up to eight regions
-                     * ago: of several walks that fail here together one
-                     * raises it, not each. (With a fresh look it rises with
-                     * every failed walk; regions with free chunks are then
-                     * passed sooner, and the refill of the 32 GiB
-                     * fragmentation run formatted 440 to 480 thousand pages
-                     * for chunks instead of 427.) */
+                    /* the counter as it was looked at, up to eight regions ago: of
+                     * several walks that fail here together one raises it */
                     level = static_cast<u32>(ahead) & 255u;
                     walking = go && level < checklevel;
                     masks = batched;
                     todo = 0u;
                     i = walking ? ~0u : R;
-                    if(walking)
+                    read = walking && batched;
+                }
+                if(read)
+                {
+                    region_candidates(h, region * R, bytes, maxchunksize, zero, todo, room);
+                    if(s0 != 0u)
                     {
-                        if(masks)
-                        {
-                            region_candidates(h, region * R, bytes, maxchunksize, zero, todo);
-                            if(s0 != 0u)
-                            {
-                                zero = ((zero >> s0) | (zero << (R - s0))) & rmask;
-                                todo = ((todo >> s0) | (todo << (R - s0))) & rmask;
-                            }
-                            todo |= zero;
-                        }
+                        zero = ((zero >> s0) | (zero << (R - s0))) & rmask;
+                        todo = ((todo >> s0) | (todo << (R - s0))) & rmask;
                     }
+                    todo = masks ? todo | zero : 0u;
+                    masks = true;
                 }
                 if(go && (masks ? todo != 0u : i + 1u < R))
                 {
@@ -699,7 +765,7 @@ namespace mmc
         {
             if(Ids::reset(h))
                 return false;
-            const u32 am = __activemask();
+            const u32 am = converged_lanes();
             const bool same = __reduce_min_sync(am, bytes) == __reduce_max_sync(am, bytes);
             const u32 peers = same ? am : __match_any_sync(am, bytes);
             const u32 k = static_cast<u32>(__popc(peers));
@@ -785,7 +851,7 @@ namespace mmc
             bool served = false;
             if constexpr(Ids::warpSize > 1u)
             {
-                const u32 am = __activemask();
+                const u32 am = converged_lanes();
                 served = claim_same_size<Ids>(h, bytes, minAllocation, maxchunksize, global_start_page, fill0, cs0, res);
                 __syncwarp(am);
             }
@@ -1258,15 +1324,518 @@ namespace mmc
             return res;
         }
 
-        /* allocPageBased, Scatter.hpp:848-866. Alone on the heap (SerialIds) this
-         * is the reference's mutex-serialised search. */
-        template<class Ids>
-        __device__ void* alloc_page_based(const mmc_device_handle& h, u32 bytes)
+        __device__ __forceinline__ void set_page_timeout(const PageScan& c)
         {
-            if(Ids::warpSize == 1u)
-                return alloc_page_based_single(h, bytes);
-            return alloc_page_based_concurrent(
-                PageScan{h.chunksize, h.freemap, h.state, h.pages, h.numpages, h.pagesize, h.reference_quirks}, bytes);
+            atomicOr(&c.state->error_flags, MMC_DEVERR_TIMEOUT);
+        }
+
+        /* ---------------------------- multi-page requests of whole warps
+         * Every concurrent search of the lock-free form above settles on the
+         * same run, the topmost that fits, and one of them gets it per round
+         * trip while all the others CAS the same word: a wave of 77 824
+         * requests on an 8 GiB heap, 7 800 of them multi-page, took 19 to
+         * 28 ms and 46 to 60 M atomics. (Served as below: 7 680 multi-page
+         * requests on an empty 8 GiB heap 55 -> 0.4 ms, among half a heap of
+         * freed and live runs 98 -> 9 ms.) Here a warp whose 32 lanes call malloc
+         * together puts its lanes' requests in a ring, and whichever waiting
+         * warp finds the lock free serves all that wait, up to 256 at a time:
+         *   - it takes the topmost free stretch at the hint for the whole
+         *     batch with one read of its bitmap words, when it is long enough;
+         *   - else it streams the bitmap down from the hint once per batch,
+         *     1024 pages at a time (a word per lane, four such windows in
+         *     flight), and gives each window's topmost run that fits to the
+         *     largest request it fits, until the window takes no more.
+         * Either is some serial order of the batch's first-fit searches, so
+         * the packing is the serial search's. The server clears the runs'
+         * bits; each asking warp then marks its own runs' chunk sizes, 32
+         * pages per instruction. Those CASes stay the authority: a run that
+         * a chunk page took a page of is put back and asked for again.
+         * Partial warps and requests above kServiceMaxPages keep the
+         * lock-free search. */
+        constexpr u32 kPageAsk = 0x80000000u; /* ring word of a waiting request */
+        constexpr u32 kPageGone = 0xC0000000u; /* ring word of a request given up */
+        constexpr u32 kPageAnswer = 0x40000000u; /* ring word of an answer: | first page */
+        constexpr u32 kPageNone = 0x3FFFFFFFu; /* answer's page when there is no run */
+        constexpr u32 kServiceMaxPages = 1024u; /* 32 claims per lane, remembered in one word */
+        constexpr u32 kServiceSlots = 8u; /* requests per lane in a batch */
+        constexpr u32 kServiceRetries = 4u; /* runs lost to chunk pages before the lock-free search is used */
+
+        __device__ __forceinline__ mmc_page_service* page_service(mmc_heap_state* state)
+        {
+            return reinterpret_cast<mmc_page_service*>(state + 1);
+        }
+
+        /* longest run of set bits in x (31 for a full word; its callers treat full words apart) */
+        __device__ __forceinline__ u32 longest_run(u32 x)
+        {
+            const u32 p1 = x & (x >> 1), p2 = p1 & (p1 >> 2), p3 = p2 & (p2 >> 4), p4 = p3 & (p3 >> 8);
+            u32 cur = ~0u, len = 0u;
+            if(p4 != 0u)
+            {
+                cur = p4;
+                len = 16u;
+            }
+            u32 c = cur & (p3 >> len);
+            if(c != 0u)
+            {
+                cur = c;
+                len += 8u;
+            }
+            c = cur & (p2 >> len);
+            if(c != 0u)
+            {
+                cur = c;
+                len += 4u;
+            }
+            c = cur & (p1 >> len);
+            if(c != 0u)
+            {
+                cur = c;
+                len += 2u;
+            }
+            c = cur & (x >> len);
+            return c != 0u ? len + 1u : len;
+        }
+
+        /* bits of word w that lie in pages [first, end) */
+        __device__ __forceinline__ u32 word_span(u32 w, u32 first, u32 end)
+        {
+            const u32 lo = umax(first, 32u * w), hi = umin(end, 32u * w + 32u);
+            if(lo >= hi)
+                return 0u;
+            const u32 n = hi - lo;
+            return n == 32u ? 0xFFFFFFFFu : ((1u << n) - 1u) << (lo & 31u);
+        }
+
+        /* One pass of a batch's requests over the windows from page `top` down
+         * to page `low` (both included), by a whole warp holding the lock.
+         * req[s] holds a request's pages, 0, or a served request's
+         * kPageAsk | first page. With `hinting`, hint receives the highest page
+         * from which a later search could still find a multi-page run. */
+        __device__ __forceinline__ void page_service_pass(const PageScan& c, u32 (&req)[kServiceSlots], u32 top, u32 low,
+                                                          bool hinting, u32& hint)
+        {
+            constexpr u32 kFull = 0xFFFFFFFFu;
+            const u32 lane = GpuIds::laneid();
+            const u32 wtop = top >> 10, wlow = low >> 10;
+            const u32 words = c.numpages / 32u + 1u;
+            u32 carry = 0u; /* free pages right above the window */
+            bool open = true; /* no usable run was left above */
+            u32 ahead[4];
+#pragma unroll
+            for(u32 k = 0; k < 4u; ++k)
+                ahead[k] = (wtop >= k && 32u * (wtop - k) + lane < words) ? ld_rlx(&c.freemap[32u * (wtop - k) + lane]) : 0u;
+            for(u32 w = wtop;; --w)
+            {
+                u32 x = ahead[0];
+                ahead[0] = ahead[1];
+                ahead[1] = ahead[2];
+                ahead[2] = ahead[3];
+                ahead[3] = w >= 4u ? ld_rlx(&c.freemap[32u * (w - 4u) + lane]) : 0u;
+                MMC_STAT_ADD(c, MMC_STAT_PAGE_SCAN, 32u);
+                x &= word_span(32u * w + lane, low, top + 1u);
+                const u32 base = 1024u * w;
+                const u32 any = __ballot_sync(kFull, x != 0u);
+                u32 pending = 0u;
+                if(any == 0u)
+                    carry = 0u;
+                else
+                {
+                    for(;;)
+                    {
+                        const u32 t = static_cast<u32>(__clz(static_cast<int>(~x)));
+                        const u32 b = x == kFull ? 32u : static_cast<u32>(__ffs(static_cast<int>(~x))) - 1u;
+                        const u32 notfull = __ballot_sync(kFull, x != kFull);
+                        /* free pages right above this lane's word */
+                        const u32 higher = lane == 31u ? 0u : notfull >> (lane + 1u);
+                        const u32 j = lane + static_cast<u32>(__ffs(static_cast<int>(higher))); /* lowest of them */
+                        const u32 bj = __shfl_sync(kFull, b, static_cast<int>(j & 31u));
+                        const u32 above = higher == 0u ? 32u * (31u - lane) + carry : 32u * (j - lane - 1u) + bj;
+                        const u32 len = longest_run(x);
+                        const u32 fit = __reduce_max_sync(kFull, umax(x != 0u ? above + t : 0u, len));
+                        /* the largest waiting request that fits */
+                        u32 mine = 0u;
+                        pending = 0u;
+#pragma unroll
+                        for(u32 s = 0; s < kServiceSlots; ++s)
+                        {
+                            const u32 v = req[s];
+                            pending |= (v != 0u && v < kPageAsk) ? 1u : 0u;
+                            mine = (v <= fit && v > mine) ? v : mine;
+                        }
+                        const u32 n = __reduce_max_sync(kFull, mine);
+                        if(n == 0u)
+                        {
+                            /* to the next window: its carry, and what this one leaves */
+                            if(open && fit > 1u)
+                            {
+                                /* the highest free page, or the stretch that joins this window's from above */
+                                open = false;
+                                const u32 hl = 31u - static_cast<u32>(__clz(static_cast<int>(__ballot_sync(kFull, x != 0u))));
+                                const u32 th = 31u - static_cast<u32>(__clz(static_cast<int>(__shfl_sync(kFull, x, static_cast<int>(hl)))));
+                                if(hinting)
+                                    hint = base + 32u * hl + th + (32u * hl + th == 1023u ? carry : 0u);
+                            }
+                            const u32 l = static_cast<u32>(__ffs(static_cast<int>(notfull))) - 1u;
+                            const u32 bl = __shfl_sync(kFull, b, static_cast<int>(l & 31u));
+                            carry = notfull == 0u ? 1024u + carry : 32u * l + bl;
+                            break;
+                        }
+                        /* its run: the topmost one */
+                        const bool crossing = x != 0u && above + t >= n;
+                        const u32 can = __ballot_sync(kFull, crossing || len >= n);
+                        const u32 src = 31u - static_cast<u32>(__clz(static_cast<int>(can)));
+                        u32 q = base + 32u * lane;
+                        if(crossing)
+                            q += 32u + above - n;
+                        else
+                        {
+                            u32 y = x;
+                            for(u32 got = 1u; got < n && y != 0u;)
+                            {
+                                const u32 d = umin(got, n - got);
+                                y &= y >> d;
+                                got += d;
+                            }
+                            q += 31u - static_cast<u32>(__clz(static_cast<int>(y)));
+                        }
+                        q = __shfl_sync(kFull, q, static_cast<int>(src));
+                        const u32 used = word_span(32u * w + lane, q, q + n);
+                        if(used != 0u)
+                        {
+                            x &= ~used;
+                            atomicAnd(&c.freemap[32u * w + lane], ~used);
+                        }
+                        if(q + n > base + 1024u)
+                        {
+                            /* the part above the window */
+                            const u32 end = (q + n - 1u) >> 5;
+                            for(u32 ww = umax(32u * w + 32u, q >> 5) + lane; ww <= end; ww += 32u)
+                                atomicAnd(&c.freemap[ww], ~word_span(ww, q, q + n));
+                            carry = 0u;
+                        }
+                        else if(q + n == base + 1024u)
+                            carry = 0u; /* the pages above, if free, no longer join this window's */
+                        const u32 who = static_cast<u32>(__ffs(static_cast<int>(__ballot_sync(kFull, mine == n)))) - 1u;
+                        bool given = lane != who;
+#pragma unroll
+                        for(u32 s = 0; s < kServiceSlots; ++s)
+                            if(!given && req[s] == n)
+                            {
+                                req[s] = kPageAsk | q;
+                                given = true;
+                            }
+                    }
+                }
+                if(any == 0u)
+                {
+#pragma unroll
+                    for(u32 s = 0; s < kServiceSlots; ++s)
+                        pending |= (req[s] != 0u && req[s] < kPageAsk) ? 1u : 0u;
+                }
+                if(hinting && open)
+                    hint = base == 0u ? 0u : umin(base - 1u, top);
+                if(w == wlow || __ballot_sync(kFull, pending != 0u) == 0u)
+                    break;
+            }
+        }
+
+        /* Serve a batch (req[s]: pages or 0); answers replace the requests as
+         * kPageAsk | first page, what found no run stays. */
+        __device__ __forceinline__ void page_service_batch(const PageScan& c, u32 (&req)[kServiceSlots])
+        {
+            constexpr u32 kFull = 0xFFFFFFFFu;
+            const u32 lane = GpuIds::laneid();
+            const u32 entry = ld_rlx(&c.state->firstFreePageBased);
+            /* the reference's wrapped hint: its searches visit no page */
+            if(entry == 0xFFFFFFFFu)
+                return;
+            const u32 start = umin(entry, c.numpages);
+            u32 mine = 0u;
+#pragma unroll
+            for(u32 s = 0; s < kServiceSlots; ++s)
+                mine += req[s];
+            const u32 sum = __reduce_add_sync(kFull, mine);
+            if(sum == 0u)
+                return;
+            /* pages (start - sum, start] all free: the batch packs there (a run at page 0 is left to the passes) */
+            if(sum < start && start < c.numpages)
+            {
+                const u32 low = start + 1u - sum;
+                bool all = true;
+                for(u32 w0 = start >> 5; all; )
+                {
+                    bool ok = true;
+#pragma unroll
+                    for(u32 k = 0; k < 4u; ++k)
+                    {
+                        const u32 off = 32u * k + lane;
+                        const u32 w = w0 - off;
+                        const u32 need = off <= w0 ? word_span(w, low, start + 1u) : 0u;
+                        if(need != 0u)
+                            MMC_STAT_ADD(c, MMC_STAT_PAGE_SCAN, 32u);
+                        if(need != 0u)
+                            ok = ok && (ld_rlx(&c.freemap[w]) & need) == need;
+                    }
+                    all = __all_sync(kFull, ok);
+                    if(w0 < 128u || 32u * (w0 - 127u) <= low)
+                        break;
+                    w0 -= 128u;
+                }
+                if(all)
+                {
+                    for(u32 w = (low >> 5) + lane; w <= (start >> 5); w += 32u)
+                        atomicAnd(&c.freemap[w], ~word_span(w, low, start + 1u));
+                    u32 incl = mine;
+#pragma unroll
+                    for(u32 off = 1u; off < 32u; off <<= 1)
+                    {
+                        const u32 v = __shfl_up_sync(kFull, incl, off);
+                        if(lane >= off)
+                            incl += v;
+                    }
+                    u32 next = start + 1u - (incl - mine);
+#pragma unroll
+                    for(u32 s = 0; s < kServiceSlots; ++s)
+                        if(req[s] != 0u)
+                        {
+                            next -= req[s];
+                            req[s] = kPageAsk | next;
+                        }
+                    if(lane == 0u)
+                        atomicCAS(&c.state->firstFreePageBased, entry, low - 1u);
+                    return;
+                }
+            }
+            /* from the hint down, then what is left from the top down to it */
+            u32 hint = start;
+#pragma unroll 1
+            for(u32 leg = 0; leg < 2u; ++leg)
+            {
+                page_service_pass(c, req, leg == 0u ? start : c.numpages, leg == 0u ? 0u : start, leg == 0u, hint);
+                bool waiting = false, at_zero = false;
+#pragma unroll
+                for(u32 s = 0; s < kServiceSlots; ++s)
+                {
+                    waiting = waiting || (req[s] != 0u && req[s] < kPageAsk);
+                    at_zero = at_zero || req[s] == kPageAsk;
+                }
+                if(leg == 0u)
+                {
+                    /* the reference stores a run's first page - 1, which wraps for a
+                     * run at page 0 (Scatter.hpp:800-804); fixed mode stores 0 */
+                    if(__any_sync(kFull, at_zero) && hint == 0u && c.reference_quirks)
+                        hint = 0xFFFFFFFFu;
+                    if(lane == 0u && hint != entry)
+                        atomicCAS(&c.state->firstFreePageBased, entry, hint);
+                }
+                if(!__any_sync(kFull, waiting))
+                    break;
+            }
+        }
+
+        /* Serve what waits in the ring, batch by batch; the caller's warp (whole) holds the lock. */
+        __device__ __noinline__ inline void page_service_run(const PageScan c)
+        {
+            constexpr u32 kFull = 0xFFFFFFFFu;
+            mmc_page_service* sv = page_service(c.state);
+            const u32 lane = GpuIds::laneid();
+            u32 head = ld_rlx(&sv->head);
+            for(u32 round = 0; round < 64u; ++round)
+            {
+                const u32 count = umin(ld_rlx(&sv->tail) - head, 32u * kServiceSlots);
+                if(__shfl_sync(kFull, count, 0) == 0u)
+                    break;
+                const u32 have = __shfl_sync(kFull, count, 0);
+                u32 req[kServiceSlots];
+                u32 taken = have;
+#pragma unroll
+                for(u32 s = 0; s < kServiceSlots; ++s)
+                {
+                    const u32 i = 32u * s + lane;
+                    req[s] = i < have ? ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]) : 0u;
+                }
+                /* a ticket drawn but not written yet (its lane is about to): the batch ends before it */
+#pragma unroll
+                for(u32 s = 0; s < kServiceSlots; ++s)
+                {
+                    const u32 i = 32u * s + lane;
+                    for(u32 spin = 0; i < taken && (req[s] & kPageAsk) == 0u; ++spin)
+                    {
+                        if(spin == 64u)
+                            taken = i;
+                        else
+                            req[s] = ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]);
+                    }
+                }
+                taken = __reduce_min_sync(kFull, taken);
+                if(taken == 0u)
+                    break;
+#pragma unroll
+                for(u32 s = 0; s < kServiceSlots; ++s)
+                {
+                    const u32 i = 32u * s + lane;
+                    if(i < taken && req[s] == kPageGone)
+                        st_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)], 0u);
+                    req[s] = (i < taken && req[s] != kPageGone) ? req[s] & ~kPageAsk : 0u;
+                }
+                u32 asked = 0u;
+#pragma unroll
+                for(u32 s = 0; s < kServiceSlots; ++s)
+                    asked |= req[s] != 0u ? 1u << s : 0u;
+                page_service_batch(c, req);
+                /* every lane's bit clears are performed before any answer is seen */
+                __threadfence();
+                __syncwarp();
+#pragma unroll
+                for(u32 s = 0; s < kServiceSlots; ++s)
+                    if((asked >> s) & 1u)
+                    {
+                        u32* word = &sv->ring[(head + 32u * s + lane) & (MMC_PAGE_RING - 1u)];
+                        st_rlx(word, kPageAnswer | ((req[s] & kPageAsk) != 0u ? req[s] & ~kPageAsk : kPageNone));
+                    }
+                head += taken;
+                if(lane == 0u)
+                    st_rlx(&sv->head, head);
+            }
+            __threadfence();
+            __syncwarp();
+            if(lane == 0u)
+                st_rlx(&sv->lock, 0u);
+        }
+
+        /* Multi-page requests of a whole warp: `bytes` per lane, 0 for none. */
+        __device__ __noinline__ inline char* alloc_page_based_warp(const PageScan c, u32 bytes)
+        {
+            constexpr u32 kFull = 0xFFFFFFFFu;
+            mmc_page_service* sv = page_service(c.state);
+            const u32 lane = GpuIds::laneid();
+            const u32 n = divup(bytes, c.pagesize);
+            bool want = n != 0u && n <= kServiceMaxPages;
+            bool search = n > kServiceMaxPages;
+            char* res = nullptr;
+            for(u32 round = 0;; ++round)
+            {
+                const u32 asking = __ballot_sync(kFull, want);
+                if(asking == 0u)
+                    break;
+                if(round == kServiceRetries)
+                {
+                    search = search || want;
+                    break;
+                }
+                u32 ticket = 0u, served = 0u;
+                if(lane == 0u)
+                {
+                    served = ld_rlx(&sv->head);
+                    ticket = atomicAdd(&sv->tail, static_cast<u32>(__popc(asking)));
+                }
+                ticket = __shfl_sync(kFull, ticket, 0) + static_cast<u32>(__popc(asking & lanemask_lt()));
+                u32* word = &sv->ring[ticket & (MMC_PAGE_RING - 1u)];
+                /* a ticket's word is its own once the ticket a whole ring
+                 * before it has been served (and, below, its answer read) */
+                bool turn = ticket - __shfl_sync(kFull, served, 0) < MMC_PAGE_RING;
+                bool written = false, waiting = want;
+                u32 q = kPageNone;
+                for(u32 it = 0;; ++it)
+                {
+                    if(waiting && !written)
+                    {
+                        if(!turn)
+                            turn = ticket - ld_rlx(&sv->head) < MMC_PAGE_RING;
+                        if(turn && ld_rlx(word) == 0u)
+                        {
+                            st_rlx(word, kPageAsk | n);
+                            written = true;
+                        }
+                        else if(it > MMC_MUTEX_MAX_SPINS)
+                        {
+                            set_page_timeout(c);
+                            waiting = false;
+                        }
+                    }
+                    else if(waiting)
+                    {
+                        const u32 v = ld_rlx(word);
+                        if((v & kPageAsk) == 0u)
+                        {
+                            q = v & kPageNone;
+                            st_rlx(word, 0u);
+                            waiting = false;
+                        }
+                        else if(it > MMC_MUTEX_MAX_SPINS && atomicCAS(word, v, kPageGone) == v)
+                        {
+                            set_page_timeout(c);
+                            waiting = false;
+                        }
+                    }
+                    if(!__any_sync(kFull, waiting))
+                        break;
+                    u32 mine = 0u;
+                    if(lane == 0u && ld_rlx(&sv->lock) == 0u)
+                        mine = atomicCAS(&sv->lock, 0u, 1u) == 0u ? 1u : 0u;
+                    if(__shfl_sync(kFull, mine, 0) != 0u)
+                    {
+                        __threadfence();
+                        page_service_run(c);
+                    }
+                    else if(it > 1u)
+                        __nanosleep(umin(64u << umin(it, 5u), 1024u));
+                }
+                /* answers are read: what the server did to the bitmap is performed before what follows */
+                __threadfence();
+                if(want && q == kPageNone)
+                {
+                    MMC_STAT(c, MMC_STAT_PAGE_BASED_FAIL);
+                    want = false;
+                }
+                /* mark the runs, the warp together */
+                for(u32 todo = __ballot_sync(kFull, want); todo != 0u; todo &= todo - 1u)
+                {
+                    const int j = __ffs(static_cast<int>(todo)) - 1;
+                    const u32 first = __shfl_sync(kFull, q, j);
+                    const u32 pages = __shfl_sync(kFull, n, j);
+                    const u32 tag = __shfl_sync(kFull, bytes, j);
+                    u32 got = 0u, lost = 0u;
+#pragma unroll 4
+                    for(u32 i = 0; i < divup(pages, 32u); ++i)
+                    {
+                        const u32 off = 32u * i + lane;
+                        const u32 old = off < pages ? atomicCAS(&c.chunksize[first + off], 0u, tag) : 0u;
+                        got |= (off < pages && old == 0u ? 1u : 0u) << i;
+                        lost |= old;
+                    }
+                    if(!__any_sync(kFull, lost != 0u))
+                    {
+                        if(lane == static_cast<u32>(j))
+                        {
+                            res = c.pages + static_cast<u64>(first) * c.pagesize;
+                            want = false;
+                        }
+                        continue;
+                    }
+                    /* A page of the run went to a chunk format or a lock-free
+                     * search: put the others back, as markpages does (each
+                     * lost page's owner keeps its bit), and ask again. */
+                    MMC_STAT(c, MMC_STAT_PAGE_LOST);
+                    u32 top = 0u;
+                    for(u32 m = got; m != 0u; m &= m - 1u)
+                    {
+                        const u32 page = first + 32u * (static_cast<u32>(__ffs(static_cast<int>(m))) - 1u) + lane;
+                        if(atomicCAS(&c.chunksize[page], tag, 0u) == tag)
+                        {
+                            freemap_set(c.freemap, page);
+                            top = page + 1u;
+                        }
+                    }
+                    if(top != 0u)
+                        atomicMax(&c.state->firstFreePageBased, top - 1u);
+                }
+                __syncwarp();
+            }
+            if(search)
+                res = alloc_page_based_concurrent(c, bytes);
+            return res;
         }
 
         /* deallocPageBased, Scatter.hpp:874-886 (out of line, as the search) */
@@ -1283,24 +1852,85 @@ namespace mmc
             atomicMax(&h.state->firstFreePageBased, page + pages - 1u);
         }
 
+        /* deallocPageBased for the lanes `runs` of the lanes `am`, which share
+         * the work: a run's page tails, chunk sizes and bitmap words spread
+         * over them. One lane alone zeroed 32 words per page and issued a
+         * CAS per page: half of a wave's 920 blocks freed on a 512 MiB heap
+         * took 202 us. The CASes have returned before the bits are set: a bit
+         * set ahead of its CAS could be taken by the server, whose claim then
+         * fails and leaves the page's bit clear for good. */
+        __device__ __noinline__ inline void dealloc_page_based_warp(const PageScan c, u32 masks, u32 am, u32 runs,
+                                                                    u32 page, u32 bytes)
+        {
+            const u32 g = static_cast<u32>(__popc(am));
+            const u32 rank = static_cast<u32>(__popc(am & lanemask_lt()));
+            for(u32 todo = runs; todo != 0u; todo &= todo - 1u)
+            {
+                const int j = __ffs(static_cast<int>(todo)) - 1;
+                const u32 first = __shfl_sync(am, page, j);
+                const u32 tag = __shfl_sync(am, bytes, j);
+                const u32 end = umin(first + divup(tag, c.pagesize), c.numpages);
+                char* tail = c.pages + static_cast<u64>(first + 1u) * c.pagesize - 4u * masks;
+                for(u32 p = first; p < end; ++p, tail += c.pagesize)
+                    for(u32 w = rank; w < masks; w += g)
+                        st_rlx(reinterpret_cast<u32*>(tail) + w, 0u);
+                __threadfence();
+                __syncwarp(am);
+                u32 old = tag;
+#pragma unroll 4
+                for(u32 p = first + rank; p < end; p += g)
+                    old &= atomicCAS(&c.chunksize[p], tag, 0u);
+                /* (old is what every lane's CASes returned: the ballot waits for them) */
+                if(__ballot_sync(am, old == tag) != 0u || old == 0u)
+                    __syncwarp(am);
+                for(u32 w = (first >> 5) + rank; 32u * w < end; w += g)
+                    atomicOr(&c.freemap[w], word_span(w, first, end));
+                if(rank == 0u)
+                    atomicMax(&c.state->firstFreePageBased, first + divup(tag, c.pagesize) - 1u);
+            }
+        }
+
         /* create, Scatter.hpp:895-912 */
         template<class Ids>
         __device__ __forceinline__ void* create(const mmc_device_handle& h, u32 bytes)
         {
+            void* res = nullptr;
+            if constexpr(Ids::pageBased && Ids::warpSize > 1u)
+            {
+                const u32 active = converged_lanes();
+                /* chunks first: a warp's chunk requests need not wait for its
+                 * multi-page ones, and in a heap that runs out they find their
+                 * last chunks before the multi-page requests take the pages (a
+                 * chunk request that finds none looks at every page, a
+                 * multi-page one at a bit per page) */
+                const bool large = bytes > h.pagesize;
+                if(bytes != 0u && !large)
+                    res = alloc_chunked<Ids>(h, bytes);
+                if(__any_sync(active, large))
+                {
+                    if(large)
+                        MMC_STAT(h, MMC_STAT_PAGE_BASED);
+                    const PageScan c{h.chunksize, h.freemap, h.state, h.pages, h.numpages, h.pagesize, h.reference_quirks};
+                    /* a whole warp's are served together */
+                    if(active == 0xFFFFFFFFu)
+                    {
+                        void* run = alloc_page_based_warp(c, large ? bytes : 0u);
+                        res = large ? run : res;
+                    }
+                    else if(large)
+                        res = alloc_page_based_concurrent(c, bytes);
+                }
+                return res;
+            }
             if(bytes == 0u)
                 return nullptr;
             if(bytes <= h.pagesize)
                 return alloc_chunked<Ids>(h, bytes);
             if constexpr(!Ids::pageBased)
-            {
                 set_error(h, MMC_DEVERR_PAGEBASED);
-                return nullptr;
-            }
             else
-            {
-                MMC_STAT(h, MMC_STAT_PAGE_BASED);
-                return alloc_page_based<Ids>(h, bytes);
-            }
+                res = alloc_page_based_single(h, bytes);
+            return res;
         }
 
         /* 64-bit division for page sizes that are not powers of two, kept out of line */
@@ -1374,24 +2004,20 @@ namespace mmc
                     return;
                 mem = counter;
             }
-            if(chunksize < P || (!h.reference_quirks && chunksize == P))
-                dealloc_chunked<Ids>(h, mem, page, chunksize);
-            else
+            const bool chunk = chunksize < P || (!h.reference_quirks && chunksize == P);
+            if constexpr(Ids::warpSize > 1u)
             {
-                if constexpr(Ids::warpSize > 1u)
-                {
-                    /* The pages are free for chunks too: the regions they lie in
-                     * are no longer as full as failed walks have counted them. The
-                     * reference leaves the counters; after an exhausted heap's
-                     * walks had raised them all, chunk walks passed the freed
-                     * pages by, and the refill of the 32 GiB fragmentation run
-                     * took 7.4 s instead of 0.9 and filled 0.7 points less. */
-                    const u32 last = umin(page + divup(chunksize, P), h.numpages) - 1u;
-                    for(u32 r = page / h.regionsize; r <= last / h.regionsize; ++r)
-                        st_rlx(&h.regions[r], 0u);
-                }
-                dealloc_page_based(h, page, chunksize);
+                const u32 am = converged_lanes();
+                const u32 runs = __ballot_sync(am, !chunk);
+                if(runs != 0u)
+                    dealloc_page_based_warp(PageScan{h.chunksize, h.freemap, h.state, h.pages, h.numpages, h.pagesize,
+                                                     h.reference_quirks},
+                                            h.maxOnPageMasks, am, runs, page, chunksize);
             }
+            else if(!chunk)
+                dealloc_page_based(h, page, chunksize);
+            if(chunk)
+                dealloc_chunked<Ids>(h, mem, page, chunksize);
         }
 
         /* OOM policy: ReturnNull::handleOOM (ReturnNull.hpp:48-51); MMC_OOM_FLAG
@@ -1419,7 +2045,7 @@ namespace mmc
             u32 active = 1u, threadcount = 0u, before = 0u, leader = 0u;
             bool coalescible = false;
             if constexpr(Ids::warpSize > 1u)
-                active = __activemask();
+                active = converged_lanes();
             const u32 lane = Ids::laneid();
             if(Ids::coalesce && Ids::distribution(h) == MMC_DIST_XMALLOCSIMD)
             {
@@ -1635,7 +2261,7 @@ namespace mmc
             u32 active = 1u, rank = 0u, nact = 1u;
             if(Ids::warpSize > 1u)
             {
-                active = __activemask();
+                active = converged_lanes();
                 nact = static_cast<u32>(__popc(active));
                 rank = static_cast<u32>(__popc(active & lanemask_lt()));
             }

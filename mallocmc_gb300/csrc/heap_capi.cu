@@ -33,6 +33,9 @@ namespace
 
     constexpr unsigned kScanThreads = 256;
     constexpr unsigned kMaxScanBlocks = 152u * 8u;
+    /* the mutable words and, right behind them, the multi-page requests' ring */
+    constexpr size_t kStateBytes = sizeof(mmc_heap_state) + sizeof(mmc_page_service);
+    static_assert(sizeof(mmc_heap_state) % 128u == 0u && kStateBytes % 128u == 0u, "lines of their own");
 
     struct SlotPartial
     {
@@ -49,7 +52,7 @@ struct mmc_heap
     bool owns_pool;
     char* pool;       /* after Shrink::alignPool */
     size_t memsize;
-    char* devblock;   /* mmc_heap_state + slot partials + result word */
+    char* devblock;   /* mmc_heap_state + mmc_page_service + slot partials + result word */
     uint32_t* freemap; /* free-page bitmap (mmc_device_handle::freemap) */
     size_t freemap_words; /* words allocated */
     mmc_heap_state* state;
@@ -431,7 +434,7 @@ namespace
         st = cuda_check(cudaMemsetAsync(h->pool + g.ptes_offset, 0, 12ull * g.numpages + 4ull * g.numregions, s),
                         "zero page table");
         if(st == MMC_OK)
-            st = cuda_check(cudaMemsetAsync(h->state, 0, sizeof(mmc_heap_state), s), "zero heap header");
+            st = cuda_check(cudaMemsetAsync(h->state, 0, kStateBytes, s), "zero heap header");
         if(st != MMC_OK)
             return st;
         const uint64_t words = static_cast<uint64_t>(g.numpages) * g.maxOnPageMasks;
@@ -496,7 +499,7 @@ namespace
         h->pool = static_cast<char*>(pool);
         h->memsize = bytes;
         align_pool(cfg->dataAlignment, &h->pool, &h->memsize);
-        const size_t devbytes = sizeof(mmc_heap_state) + sizeof(SlotPartial) * kMaxScanBlocks + 128u;
+        const size_t devbytes = kStateBytes + sizeof(SlotPartial) * kMaxScanBlocks + 128u;
         if(cudaMalloc(&h->devblock, devbytes) != cudaSuccess
            || cudaMallocHost(reinterpret_cast<void**>(&h->host_result), sizeof(unsigned)) != cudaSuccess)
         {
@@ -509,8 +512,8 @@ namespace
             return fail(MMC_ERR_OOM, "cudaMalloc of the heap header failed");
         }
         h->state = reinterpret_cast<mmc_heap_state*>(h->devblock);
-        h->partials = reinterpret_cast<SlotPartial*>(h->devblock + sizeof(mmc_heap_state));
-        h->result_word = reinterpret_cast<unsigned*>(h->devblock + sizeof(mmc_heap_state)
+        h->partials = reinterpret_cast<SlotPartial*>(h->devblock + kStateBytes);
+        h->result_word = reinterpret_cast<unsigned*>(h->devblock + kStateBytes
                                                      + sizeof(SlotPartial) * kMaxScanBlocks);
         st = init_heap(h, s);
         if(st != MMC_OK)

@@ -165,25 +165,26 @@ __device__ __forceinline__ uint32_t warp_pattern(char* ptr, uint32_t bytes, uint
     return bad;
 }
 
-/* Uniform stress: sizes[r * nthreads + t] or drawn from the seed. Launch
- * bounds of four 256-thread CTAs per SM (64 registers): that build measured
- * about 6 % faster on GB300 than the one without the bound. With the warp
- * pattern, each verified block's whole cache lines are dropped from L2
- * (discard_dead_block) before it is freed: the block is dead, and its
- * payload would otherwise be written back to DRAM (6 % faster). */
-template<uint32_t PATTERN, class Ids>
-__global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h, mmc_stress_params p,
-                                                         const uint16_t* sizes, unsigned long long* stats)
+/* What a stress thread counts. 32 bits where a thread counts at most `rounds`
+ * pairs: at the kernel's 64-register bound every register the loop keeps live
+ * is one the allocator need not spill. */
+struct StressCounts
 {
-    /* 32-bit thread index and per-thread counts (a thread counts at most
-     * `rounds` pairs): at the kernel's 64-register bound every register the
-     * loop keeps live is one the allocator need not spill */
+    uint32_t pairs, nulls, bad;
+    unsigned long long csum, other; /* other: the checksum of lane ^ 16 (warp_pattern) */
+};
+
+/* A thread's rounds of malloc, pattern, free. With the warp pattern, each
+ * verified block's whole cache lines are dropped from L2 (discard_dead_block)
+ * before it is freed: the block is dead, and its payload would otherwise be
+ * written back to DRAM (6 % faster). */
+template<uint32_t PATTERN, class Ids>
+__device__ __forceinline__ void stress_rounds(const mmc_device_handle& h, const mmc_stress_params& p,
+                                              const uint16_t* sizes, PatternPieces* pieces, StressCounts& n)
+{
     const uint32_t nthreads = gridDim.x * blockDim.x;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nsizes = (p.hi - p.lo) / p.step + 1u;
-    uint32_t pairs = 0, nulls = 0, bad = 0;
-    unsigned long long csum = 0, other = 0;
-    __shared__ PatternPieces pieces[PATTERN == MMC_PATTERN_WARP ? 8 : 1]; /* a warp's each */
     for(uint32_t r = 0; r < p.rounds; ++r)
     {
         const uint64_t m = mix64(p.seed, t, r);
@@ -193,47 +194,95 @@ __global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h,
         if constexpr(PATTERN == MMC_PATTERN_WARP)
         {
             /* every lane takes part, with or without a block */
-            bad += warp_pattern(ptr, bytes, m, csum, other, pieces[threadIdx.x / 32u]);
+            n.bad += warp_pattern(ptr, bytes, m, n.csum, n.other, pieces[threadIdx.x / 32u]);
             if(ptr == nullptr)
-                ++nulls;
+                ++n.nulls;
             else
             {
                 /* the verified block is dead: its whole lines leave L2 unwritten */
                 dv::free<Ids>(h, dv::discard_dead_block(ptr, bytes));
-                ++pairs;
+                ++n.pairs;
             }
             continue;
         }
         if(ptr == nullptr)
         {
-            ++nulls;
+            ++n.nulls;
             continue;
         }
         if constexpr(PATTERN == MMC_PATTERN_THREAD)
-        {
-            thread_pattern<2>(ptr, bytes, m, bad, csum);
-        }
+            thread_pattern<2>(ptr, bytes, m, n.bad, n.csum);
         dv::free<Ids>(h, ptr);
-        ++pairs;
+        ++n.pairs;
     }
+}
+
+/* The rounds of a warp that asks for more than a page now and then: out of
+ * line, the kernel's common rounds keep their registers. */
+template<uint32_t PATTERN, class Ids>
+__device__ __noinline__ StressCounts stress_rounds_large(const mmc_device_handle h, const mmc_stress_params p,
+                                                         const uint16_t* sizes, PatternPieces* pieces)
+{
+    StressCounts n{};
+    stress_rounds<PATTERN, Ids>(h, p, sizes, pieces, n);
+    return n;
+}
+
+/* malloc of a warp with a multi-page request among its lanes', out of line for the same reason */
+template<class Ids>
+__device__ __noinline__ void* malloc_large(const mmc_device_handle h, uint32_t bytes)
+{
+    return dv::malloc<Ids>(h, bytes);
+}
+
+/* Uniform stress: sizes[r * nthreads + t] or drawn from the seed. Launch
+ * bounds of four 256-thread CTAs per SM (64 registers): that build measured
+ * about 6 % faster on GB300 than the one without the bound.
+ *
+ * A warp whose requests all fit a page, the usual one, runs its rounds without
+ * the multi-page path: with the call of it in the loop ptxas spilled 172 bytes
+ * at that bound (5.92 against 4.97 ms on the uniform stress), and with both
+ * loops inlined 252 (5.52 ms). It looks the
+ * size table through first, when there is one, 200 bytes a thread of the
+ * benchmark's. */
+template<uint32_t PATTERN, class Ids>
+__global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h, mmc_stress_params p,
+                                                         const uint16_t* sizes, unsigned long long* stats)
+{
+    __shared__ PatternPieces pieces[PATTERN == MMC_PATTERN_WARP ? 8 : 1]; /* a warp's each */
+    uint32_t most = p.hi;
+    if(sizes != nullptr)
+    {
+        const uint32_t nthreads = gridDim.x * blockDim.x;
+        const uint16_t* mine = sizes + blockIdx.x * blockDim.x + threadIdx.x;
+        most = 0u;
+#pragma unroll 8
+        for(uint32_t r = 0; r < p.rounds; ++r)
+            most = max(most, static_cast<uint32_t>(mine[static_cast<uint64_t>(r) * nthreads]));
+    }
+    StressCounts n{};
+    if(__any_sync(__activemask(), dv::apply_padding(Ids::alignment(h), most) > h.pagesize))
+        n = stress_rounds_large<PATTERN, Ids>(h, p, sizes, pieces);
+    else
+        stress_rounds<PATTERN, dv::SmallRequests<Ids>>(h, p, sizes, pieces, n);
     if constexpr(PATTERN == MMC_PATTERN_WARP)
-        csum += __shfl_xor_sync(0xFFFFFFFFu, other, 16);
+        n.csum += __shfl_xor_sync(0xFFFFFFFFu, n.other, 16);
     /* warp-aggregate the counters */
     for(int off = 16; off > 0; off >>= 1)
     {
-        pairs += __shfl_down_sync(0xFFFFFFFFu, pairs, off);
-        nulls += __shfl_down_sync(0xFFFFFFFFu, nulls, off);
-        bad += __shfl_down_sync(0xFFFFFFFFu, bad, off);
-        csum ^= __shfl_down_sync(0xFFFFFFFFu, csum, off);
+        n.pairs += __shfl_down_sync(0xFFFFFFFFu, n.pairs, off);
+        n.nulls += __shfl_down_sync(0xFFFFFFFFu, n.nulls, off);
+        n.bad += __shfl_down_sync(0xFFFFFFFFu, n.bad, off);
+        n.csum ^= __shfl_down_sync(0xFFFFFFFFu, n.csum, off);
     }
     if((threadIdx.x & 31u) == 0u)
     {
-        atomicAdd(&stats[0], static_cast<unsigned long long>(pairs));
-        if(nulls)
-            atomicAdd(&stats[1], static_cast<unsigned long long>(nulls));
-        if(bad)
-            atomicAdd(&stats[2], static_cast<unsigned long long>(bad));
-        atomicXor(&stats[3], csum);
+        atomicAdd(&stats[0], static_cast<unsigned long long>(n.pairs));
+        if(n.nulls)
+            atomicAdd(&stats[1], static_cast<unsigned long long>(n.nulls));
+        if(n.bad)
+            atomicAdd(&stats[2], static_cast<unsigned long long>(n.bad));
+        atomicXor(&stats[3], n.csum);
     }
 }
 
@@ -340,8 +389,10 @@ __device__ __forceinline__ unsigned long long frag_check_tags(const char* p, uin
     return bad;
 }
 
+/* Bounded to 64 registers, four blocks per SM: unbounded, the multi-page
+ * service takes 103 and two blocks fit. */
 template<class Ids>
-__global__ void __launch_bounds__(256) mmc_fill_kernel(mmc_device_handle h, mmc_frag_params p, uint64_t wave,
+__global__ void __launch_bounds__(256, 4) mmc_fill_kernel(mmc_device_handle h, mmc_frag_params p, uint64_t wave,
                                                        void** ptrs, uint32_t* sizes, uint64_t capacity,
                                                        unsigned long long* counters)
 {
@@ -406,9 +457,11 @@ __global__ void mmc_verify_list_kernel(void* const* ptrs, const uint32_t* sizes,
         atomicAdd(&counters[3], bad);
 }
 
-/* Verify workload: malloc(sizes[t]); write u32 (t ^ seed); optionally verify and free. */
+/* Verify workload: malloc(sizes[t]); write u32 (t ^ seed); optionally verify
+ * and free. Bounded to 64 registers (blocks of up to 1024 threads): unbounded,
+ * the multi-page service takes 105. */
 template<bool ALLOC, bool FREE, class Ids>
-__global__ void mmc_verify_kernel(mmc_device_handle h, uint32_t nthreads, const uint32_t* sizes, uint32_t seed,
+__global__ void __launch_bounds__(1024) mmc_verify_kernel(mmc_device_handle h, uint32_t nthreads, const uint32_t* sizes, uint32_t seed,
                                   int64_t* offsets, unsigned long long* errors)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -419,7 +472,11 @@ __global__ void mmc_verify_kernel(mmc_device_handle h, uint32_t nthreads, const 
     uint32_t* p = nullptr;
     if(ALLOC)
     {
-        p = static_cast<uint32_t*>(dv::malloc<Ids>(h, sizes[t]));
+        /* warps whose requests all fit a page keep clear of the multi-page path (see the stress kernel) */
+        if(__any_sync(__activemask(), dv::apply_padding(Ids::alignment(h), sizes[t]) > h.pagesize))
+            p = static_cast<uint32_t*>(malloc_large<Ids>(h, sizes[t]));
+        else
+            p = static_cast<uint32_t*>(dv::malloc<dv::SmallRequests<Ids>>(h, sizes[t]));
         offsets[t] = p ? static_cast<int64_t>(reinterpret_cast<char*>(p) - h.pages) : -1;
         if(p)
             for(uint32_t i = 0; i < sizes[t] / 4u; ++i)
@@ -534,10 +591,7 @@ mmc_status mmc_run_stress(mmc_heap* heap, const mmc_stress_params* p, const uint
         return fail(MMC_ERR_ARG, "stress grid above 2^32 threads or more than 2^26 rounds");
     mmc_device_handle h;
     mmc_heap_device_handle(heap, &h);
-    /* One instantiation per pattern mode: only the mode's code is in the
-     * kernel. It keeps the multi-page path even when hi fits a page: built
-     * without it (SmallRequests) the uniform stress measured 1.5 % slower on
-     * GB300, from a different allocation of its 64 registers. */
+    /* One instantiation per pattern mode: only the mode's code is in the kernel. */
     MMC_DISPATCH_IDS(h, if(p->write_pattern == MMC_PATTERN_WARP) mmc_stress_kernel<MMC_PATTERN_WARP, Ids>
                             <<<p->blocks, p->threads_per_block, 0, as_stream(stream)>>>(h, *p, sizes, stats);
                      else mmc_stress_kernel<MMC_PATTERN_THREAD, Ids>

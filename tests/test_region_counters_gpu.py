@@ -1,35 +1,42 @@
-"""A multi-page free resets the counters of the regions its pages lie in: after
-chunk walks have found a full heap and raised every region's counter, chunks
-are served again from the freed run's pages, wherever in the heap they are."""
+"""The region counters under concurrent ids: a walk that finds nothing counts in
+regions with no page and no chunk free, and leaves those alone that have room
+for another size; the heap's second pass counts nowhere."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("pages", [2, 15, 16, 17, 40])
-def test_multi_page_free_opens_its_regions(pages):
+@pytest.mark.parametrize("regionsize", [8, 16, 32])
+def test_failed_walks_count_in_full_regions_only(regionsize):
     from mallocmc_gb300 import Allocator
     from mallocmc_gb300.policies import CreationPolicies
     from mallocmc_gb300.workloads import alloc_offsets, free_offsets
 
-    with Allocator(CreationPolicies.Scatter(accessblocksize=8 << 20), size=32 << 20) as alloc:
+    with Allocator(CreationPolicies.Scatter(accessblocksize=8 << 20, regionsize=regionsize),
+                   size=32 << 20) as alloc:
         total = alloc.geometry().numpages
-        size = np.array([pages * 4096], dtype=np.uint32)
-        runs = [alloc_offsets(alloc, 1, 1, size, i) for i in range(4)]
-        first = [int(o.cpu().item()) // 4096 for _, o in runs]
-        assert min(first) >= 0
-        # every other page formatted for 2048-byte chunks, and more requests than fit
-        n = 2 * (total - 4 * pages) + 64
-        _, offs = alloc_offsets(alloc, -(-n // 32), 32, np.full(-(-n // 32) * 32, 2048, dtype=np.uint32), 9)
-        assert int((offs >= 0).sum().item()) == 2 * (total - 4 * pages)
-        regions = alloc.snapshot()[1]
-        lo, hi = first[2] // 16, (first[2] + pages - 1) // 16
-        # a failing walk raises every region it leaves (of several at once, one does)
-        assert np.all(regions[lo: hi + 1] >= 1)
-        assert free_offsets(alloc, 1, 1, *runs[2], 2) == 0
-        ptes, regions, _, _ = alloc.snapshot()
-        assert np.all(regions[lo: hi + 1] == 0) and np.all(ptes[first[2]: first[2] + pages, 0] == 0)
-        _, again = alloc_offsets(alloc, 1, 1, np.array([2048], dtype=np.uint32), 10)
-        assert first[2] <= int(again.cpu().item()) // 4096 < first[2] + pages
+        n = 2 * total
+        ds, offs = alloc_offsets(alloc, n // 32, 32, np.full(n, 2048, dtype=np.uint32), 1)
+        pages = offs.cpu().numpy() // 4096
+        assert pages.min() >= 0  # two chunks on every page
+        # one chunk back on every 200th page
+        victims = np.isin(pages, np.arange(0, total, 200)) & (offs.cpu().numpy() % 4096 == 0)
+        import torch
+
+        part = torch.where(torch.from_numpy(victims).cuda(), offs, torch.full_like(offs, -1))
+        assert free_offsets(alloc, n // 32, 32, ds, part, 1) == 0
+        before = alloc.snapshot()[1].astype(np.int64)
+        for seed in range(3):  # a whole page: no region has one, many have room for less
+            _, got = alloc_offsets(alloc, 1, 1, np.array([4096], dtype=np.uint32), seed)
+            assert int(got.cpu().item()) == -1
+        after = alloc.snapshot()[1].astype(np.int64)
+        room = np.zeros(len(before), dtype=bool)
+        room[np.arange(0, total, 200) // regionsize] = True
+        assert np.array_equal(after[room], before[room])
+        level = 3 * regionsize // 4
+        assert np.array_equal(after[~room], np.where(before[~room] < level, np.minimum(before[~room] + 3, level),
+                                                     before[~room]))
+        _, again = alloc_offsets(alloc, 1, 1, np.array([2048], dtype=np.uint32), 5)
+        assert int(again.cpu().item()) // 4096 % 200 == 0
         assert alloc.error_flags() == 0
