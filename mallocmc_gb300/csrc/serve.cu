@@ -309,16 +309,9 @@ __global__ void __launch_bounds__(kCountThreads)
 {
     constexpr uint32_t nwarps = kCountThreads / 32u;
     const uint32_t np = h.numpages;
-    const uint32_t per_block = (np + gridDim.x - 1u) / gridDim.x;
+    const uint32_t per_block = ((np + gridDim.x - 1u) / gridDim.x + 3u) & ~3u;
     const uint32_t b0 = min(blockIdx.x * per_block, np);
-    const uint32_t b1 = min(b0 + per_block, np);
-    const uint32_t maxchunksize = dv::umin(h.pagesize, h.wastefactor * slot);
-    const uint32_t slotChunk = dv::umax(slot, h.paddedMinChunkSize);
-    const uint32_t capSlotChunk = dv::page_capacity(h, slotChunk);
-    uint32_t sum = 0u;
-    for(uint32_t pg = b0 + threadIdx.x; pg < b1; pg += kCountThreads)
-        sum += dv::page_free_slots(h, __ldcg(&h.chunksize[pg]), __ldcg(&h.count[pg]), slot, maxchunksize, slotChunk,
-                                   capSlotChunk);
+    uint32_t sum = free_slots_of_range(h, slot, b0, min(b0 + per_block, np), kCountThreads);
     __shared__ uint32_t ws[nwarps];
     __shared__ bool last;
     sum = __reduce_add_sync(0xFFFFFFFFu, sum);
