@@ -28,6 +28,7 @@
  */
 #include "mmc_internal.h"
 
+#include <algorithm>
 #include <cstring>
 #include <new>
 #include <string>
@@ -116,6 +117,7 @@ __global__ void mmc_serve_apply(mmc_serve_slot* slots, mmc_serve_slot* mirror, c
                                 const uint32_t* qlen, uint32_t queue_cap, uint32_t nslots, uint32_t max_len,
                                 uint32_t* error_flags)
 {
+    await_previous();
     uint32_t n = *qlen;
     if(n > queue_cap)
     {
@@ -149,7 +151,10 @@ __global__ void mmc_serve_apply(mmc_serve_slot* slots, mmc_serve_slot* mirror, c
     }
 }
 
-/* Grow one live request by `step` elements (one warp), completing it at its length. */
+/* Grow one live request by `step` elements (one warp), completing it at its
+ * length. Every lane holds the slot's values and leaves with the new ones: a
+ * tick is a chain of round trips, and reading the slot once, and a chunk's
+ * pointer from the lane that allocated it, takes three of them out. */
 template<class Ids>
 __device__ __forceinline__ void grow_request(const mmc_device_handle& h, mmc_serve_slot& s, void** chunks,
                                              uint32_t max_chunks, uint32_t step)
@@ -161,21 +166,33 @@ __device__ __forceinline__ void grow_request(const mmc_device_handle& h, mmc_ser
     /* chunks this step needs: one per 256-element boundary crossed */
     const uint32_t first_chunk = (len + kElemsPerChunk - 1u) / kElemsPerChunk;
     const uint32_t last_chunk = (end + kElemsPerChunk - 1u) / kElemsPerChunk; /* exclusive */
-    for(uint32_t c = first_chunk + lane; c < last_chunk && c < max_chunks; c += 32u)
+    const bool inside = len % kElemsPerChunk != 0u; /* elements go into the last chunk first */
+    void* tail = inside ? chunks[len / kElemsPerChunk] : nullptr;
+    void* fresh = nullptr; /* the lane's chunk of the first 32 */
+    if(first_chunk < last_chunk)
     {
-        void* p = dv::malloc<Ids>(h, kChunkBytes);
-        chunks[c] = p;
-        failed += p == nullptr;
+        for(uint32_t c = first_chunk + lane; c < last_chunk && c < max_chunks; c += 32u)
+        {
+            void* p = dv::malloc<Ids>(h, kChunkBytes);
+            chunks[c] = p;
+            fresh = c < first_chunk + 32u ? p : fresh;
+            failed += p == nullptr;
+        }
+        failed = __reduce_add_sync(0xFFFFFFFFu, failed);
+        if(!inside)
+            tail = reinterpret_cast<void*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(fresh), 0));
+        __syncwarp();
     }
-    failed = __reduce_add_sync(0xFFFFFFFFu, failed);
-    __syncwarp();
     if(failed == 0u)
     {
         for(uint32_t e = len + lane; e < end; e += 32u)
         {
-            uint16_t* chunk = static_cast<uint16_t*>(chunks[e / kElemsPerChunk]);
+            const uint32_t c = e / kElemsPerChunk;
+            uint16_t* chunk = static_cast<uint16_t*>(c == len / kElemsPerChunk ? tail : chunks[c]);
             chunk[e % kElemsPerChunk] = static_cast<uint16_t>(mix64(s.seed, e, 0x5E7ull));
         }
+        s.len = end;
+        s.nchunks = last_chunk;
     }
     else
     {
@@ -183,17 +200,7 @@ __device__ __forceinline__ void grow_request(const mmc_device_handle& h, mmc_ser
         for(uint32_t c = first_chunk + lane; c < last_chunk && c < max_chunks; c += 32u)
             if(chunks[c])
                 dv::free<Ids>(h, chunks[c]);
-    }
-    __syncwarp();
-    if(lane == 0u)
-    {
-        if(failed)
-            s.failed += 1u;
-        else
-        {
-            s.len = end;
-            s.nchunks = last_chunk;
-        }
+        s.failed += 1u;
     }
     __syncwarp();
     if(failed == 0u && end == s.final_len)
@@ -201,24 +208,37 @@ __device__ __forceinline__ void grow_request(const mmc_device_handle& h, mmc_ser
         /* complete: read every element back, checksum, free the chunks. A
          * chunk's 256 elements are 512 contiguous bytes (at the chunk's
          * 16-byte aligned start), one 16-byte load per lane: the warp reads a
-         * chunk per instruction, four chunks in flight, instead of 64 bytes
-         * per instruction element by element. Bytes past the request's last
-         * element lie inside its last chunk and are not summed. */
+         * chunk per instruction, eight chunks in flight, their pointers read
+         * 32 at a time. Bytes past the request's last element lie inside its
+         * last chunk and are not summed. */
         unsigned long long sum = 0ull;
-        const uint32_t nch = (end + kElemsPerChunk - 1u) / kElemsPerChunk;
-#pragma unroll 4
-        for(uint32_t c = 0; c < nch; ++c)
+        for(uint32_t c0 = 0; c0 < last_chunk; c0 += 32u)
         {
-            const uint4 v = reinterpret_cast<const uint4*>(chunks[c])[lane];
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-            const uint32_t e0 = c * kElemsPerChunk + lane * 8u;
-#pragma unroll
-            for(uint32_t k = 0; k < 8u; ++k)
+            const uint32_t nch = min(last_chunk - c0, 32u);
+            const unsigned long long mine = lane < nch ? reinterpret_cast<unsigned long long>(chunks[c0 + lane]) : 0ull;
+#pragma unroll 1
+            for(uint32_t k = 0; k < nch; k += 8u)
             {
-                const uint32_t e = e0 + k;
-                const uint32_t x = (w[k / 2u] >> (16u * (k & 1u))) & 0xFFFFu;
-                if(e < end)
-                    sum += static_cast<unsigned long long>(x) * (e + 1ull);
+                uint4 v[8];
+#pragma unroll
+                for(uint32_t j = 0; j < 8u; ++j)
+                {
+                    const unsigned long long p = __shfl_sync(0xFFFFFFFFu, mine, static_cast<int>((k + j) & 31u));
+                    v[j] = k + j < nch ? reinterpret_cast<const uint4*>(p)[lane] : make_uint4(0u, 0u, 0u, 0u);
+                }
+#pragma unroll
+                for(uint32_t j = 0; j < 8u; ++j)
+                {
+                    const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+                    const uint32_t e0 = (c0 + k + j) * kElemsPerChunk + lane * 8u;
+#pragma unroll
+                    for(uint32_t b = 0; b < 8u; ++b)
+                    {
+                        const uint32_t x = (w[b / 2u] >> (16u * (b & 1u))) & 0xFFFFu;
+                        if(e0 + b < end)
+                            sum += static_cast<unsigned long long>(x) * (e0 + b + 1ull);
+                    }
+                }
             }
         }
         for(int off = 16; off > 0; off >>= 1)
@@ -226,15 +246,15 @@ __device__ __forceinline__ void grow_request(const mmc_device_handle& h, mmc_ser
         __syncwarp();
         for(uint32_t c = lane; c < last_chunk; c += 32u)
             dv::free<Ids>(h, chunks[c]);
-        if(lane == 0u)
-        {
-            s.checksum = sum;
-            s.state = MMC_SERVE_DONE;
-        }
+        s.checksum = sum; /* lane 0's is the request's */
+        s.state = MMC_SERVE_DONE;
     }
 }
 
-/* Batched tick: one warp per slot; each grown slot is written to the host's
+/* Batched tick: one warp per slot, in blocks of two warps (the slots' work
+ * differs, and a block's place is taken when its last warp ends: a burst's tick
+ * 18.6 us against 19.5 in blocks of eight; bounded to 64 registers, the kernel
+ * spills and the tick takes 21); each grown slot is written to the host's
  * table. With `done` (pipelined ticks), a request that completes here is also
  * appended to the completion list, and each request still live adds the chunks
  * it will yet take to counts[1] (counts[0] is the list's length). */
@@ -244,16 +264,18 @@ __global__ void __launch_bounds__(256) mmc_serve_tick_kernel(mmc_device_handle h
                                                              uint32_t max_chunks, uint32_t step,
                                                              mmc_serve_done* done, unsigned long long* counts)
 {
+    await_previous();
     const uint32_t warps = gridDim.x * (blockDim.x / 32u);
     for(uint32_t w = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; w < nslots; w += warps)
     {
         if(slots[w].state != MMC_SERVE_LIVE)
             continue;
-        grow_request<Ids>(h, slots[w], chunks + static_cast<uint64_t>(w) * max_chunks, max_chunks, step);
+        mmc_serve_slot sw = slots[w];
+        grow_request<Ids>(h, sw, chunks + static_cast<uint64_t>(w) * max_chunks, max_chunks, step);
         __syncwarp();
         if((threadIdx.x & 31u) == 0u)
         {
-            const mmc_serve_slot sw = slots[w];
+            slots[w] = sw;
             mirror[w] = sw;
             if(done != nullptr)
             {
@@ -277,6 +299,7 @@ __global__ void __launch_bounds__(256) mmc_serve_tick_kernel(mmc_device_handle h
 __global__ void mmc_serve_publish(const mmc_serve_done* done, unsigned long long* counts, mmc_serve_done* out,
                                   uint32_t* out_len, unsigned long long* out_remaining)
 {
+    await_previous();
     const uint32_t n = static_cast<uint32_t>(counts[0]);
     for(uint32_t i = threadIdx.x; i < n; i += blockDim.x)
         out[i] = done[i];
@@ -307,6 +330,7 @@ __global__ void __launch_bounds__(kCountThreads)
                     const mmc_serve_done* done, unsigned long long* counts, mmc_serve_done* out, uint32_t* out_len,
                     unsigned long long* out_remaining)
 {
+    await_previous();
     constexpr uint32_t nwarps = kCountThreads / 32u;
     const uint32_t np = h.numpages;
     const uint32_t per_block = ((np + gridDim.x - 1u) / gridDim.x + 3u) & ~3u;
@@ -368,12 +392,16 @@ template<class Ids>
 __global__ void mmc_serve_one_kernel(mmc_device_handle h, mmc_serve_slot* slots, mmc_serve_slot* mirror,
                                      void** chunks, uint32_t slot, uint32_t max_chunks, uint32_t step)
 {
-    if(slots[slot].state != MMC_SERVE_LIVE)
+    mmc_serve_slot s = slots[slot];
+    if(s.state != MMC_SERVE_LIVE)
         return;
-    grow_request<Ids>(h, slots[slot], chunks + static_cast<uint64_t>(slot) * max_chunks, max_chunks, step);
+    grow_request<Ids>(h, s, chunks + static_cast<uint64_t>(slot) * max_chunks, max_chunks, step);
     __syncwarp();
     if(threadIdx.x == 0u)
-        mirror[slot] = slots[slot];
+    {
+        slots[slot] = s;
+        mirror[slot] = s;
+    }
 }
 
 namespace
@@ -438,56 +466,54 @@ namespace
         return MMC_OK;
     }
 
-    /* The tick's stream work: queue upload, apply, grow (batched) or not,
-     * free-slot count, slot table and count download. */
-    mmc_status enqueue_tick(mmc_server* s, bool batched)
+    /* A tick's kernels in its stream: apply the queue, grow (batched), count
+     * the free chunks into *free_out, and for a pipelined tick (p) publish its
+     * completions. Each is launched ahead of the end of the one before
+     * (launch_after), also where the stream is captured into the tick's graph. */
+    mmc_status enqueue_tick_kernels(mmc_server* s, const mmc_serve_cmd* queue, const uint32_t* queue_len,
+                                    unsigned* free_out, mmc_server::Pipe* p)
     {
         cudaStream_t st = s->stream;
-        mmc_serve_apply<<<8, 128, 0, st>>>(s->d_slots, s->m_slots, s->m_queue, s->m_queue_len, s->queue_cap, s->slots,
-                                           max_request_len(s), &s->handle.state->error_flags);
-        if(batched)
-        {
-            const uint32_t blocks = (s->slots + 7u) / 8u;
-            MMC_DISPATCH_IDS_SIZED(s->handle, kChunkBytes, mmc_serve_tick_kernel<Ids><<<blocks, 256, 0, st>>>(
-                                            s->handle, s->d_slots, s->m_slots, s->d_chunks, s->slots, s->max_chunks,
-                                            s->step, nullptr, nullptr));
-        }
+        cudaError_t e = launch_after(mmc_serve_apply, 8u, 128u, st, s->d_slots, s->m_slots, queue, queue_len,
+                                     s->queue_cap, s->slots, max_request_len(s), &s->handle.state->error_flags);
+        mmc_serve_done* done = p != nullptr ? p->d_done : nullptr;
+        unsigned long long* counts = p != nullptr ? p->d_counts : nullptr;
+        if(e == cudaSuccess)
+            MMC_DISPATCH_IDS_SIZED(s->handle, kChunkBytes,
+                                   e = launch_after(mmc_serve_tick_kernel<Ids>, (s->slots + 1u) / 2u, 64u, st, s->handle,
+                                                    s->d_slots, s->m_slots, s->d_chunks, s->slots, s->max_chunks,
+                                                    s->step, done, counts));
+        if(e != cudaSuccess)
+            return cuda_check(e, "serve tick");
         if(kChunkBytes < s->handle.pagesize)
-            mmc_serve_count<false><<<s->count_blocks, kCountThreads, 0, st>>>(
-                s->handle, kChunkBytes, s->d_count_partials, s->d_count_arrived, s->m_free, nullptr, nullptr, nullptr,
-                nullptr, nullptr);
-        else
         {
-            mmc_status r = mmc_available_slots_async(s->heap, kChunkBytes, st, s->m_free);
-            if(r != MMC_OK)
-                return r;
+            if(p != nullptr)
+                e = launch_after(mmc_serve_count<true>, s->count_blocks, kCountThreads, st, s->handle, kChunkBytes,
+                                 s->d_count_partials, s->d_count_arrived, free_out, done, counts, p->m_done,
+                                 p->m_done_len, p->m_remaining);
+            else
+                e = launch_after(mmc_serve_count<false>, s->count_blocks, kCountThreads, st, s->handle, kChunkBytes,
+                                 s->d_count_partials, s->d_count_arrived, free_out, nullptr, nullptr, nullptr, nullptr,
+                                 nullptr);
+            return cuda_check(e, "serve tick");
         }
-        return cuda_check(cudaGetLastError(), "serve tick");
+        mmc_status r = mmc_available_slots_async(s->heap, kChunkBytes, st, free_out);
+        if(r == MMC_OK && p != nullptr)
+            r = cuda_check(launch_after(mmc_serve_publish, 1u, 256u, st, done, counts, p->m_done, p->m_done_len,
+                                        p->m_remaining),
+                           "publish tick");
+        return r;
     }
-    /* A pipelined tick on buffer b: apply its queue, grow, count the free
-     * chunks into its mapped count, publish its completions. */
+
+    mmc_status enqueue_tick(mmc_server* s)
+    {
+        return enqueue_tick_kernels(s, s->m_queue, s->m_queue_len, s->m_free, nullptr);
+    }
+
     mmc_status enqueue_pipelined_tick(mmc_server* s, int b)
     {
-        cudaStream_t st = s->stream;
         mmc_server::Pipe& p = s->pipe[b];
-        mmc_serve_apply<<<8, 128, 0, st>>>(s->d_slots, s->m_slots, p.m_queue, p.m_queue_len, s->queue_cap, s->slots,
-                                           max_request_len(s), &s->handle.state->error_flags);
-        const uint32_t blocks = (s->slots + 7u) / 8u;
-        MMC_DISPATCH_IDS_SIZED(s->handle, kChunkBytes, mmc_serve_tick_kernel<Ids><<<blocks, 256, 0, st>>>(
-                                        s->handle, s->d_slots, s->m_slots, s->d_chunks, s->slots, s->max_chunks,
-                                        s->step, p.d_done, p.d_counts));
-        if(kChunkBytes < s->handle.pagesize)
-            mmc_serve_count<true><<<s->count_blocks, kCountThreads, 0, st>>>(
-                s->handle, kChunkBytes, s->d_count_partials, s->d_count_arrived, p.m_free, p.d_done, p.d_counts,
-                p.m_done, p.m_done_len, p.m_remaining);
-        else
-        {
-            mmc_status r = mmc_available_slots_async(s->heap, kChunkBytes, st, p.m_free);
-            if(r != MMC_OK)
-                return r;
-            mmc_serve_publish<<<1, 256, 0, st>>>(p.d_done, p.d_counts, p.m_done, p.m_done_len, p.m_remaining);
-        }
-        return cuda_check(cudaGetLastError(), "pipelined serve tick");
+        return enqueue_tick_kernels(s, p.m_queue, p.m_queue_len, p.m_free, &p);
     }
 
     /* cudaHostAlloc(mapped) + its device address */
@@ -550,7 +576,8 @@ mmc_status mmc_serve_create(mmc_heap* heap, uint32_t slots, uint32_t max_chunks,
     if(st == MMC_OK)
         st = cuda_check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->m_free), s->h_free, 0),
                         "mapped free count");
-    s->count_blocks = scan_grid(s->device);
+    /* 1024 pages a block: more blocks only add arrivals to the last one's wait */
+    s->count_blocks = std::max(1u, std::min(scan_grid(s->device), (s->handle.numpages + 1023u) / 1024u));
     if(st == MMC_OK)
         st = cuda_check(cudaMalloc(&s->d_count_partials, sizeof(uint32_t) * s->count_blocks), "count partials");
     if(st == MMC_OK)
@@ -574,7 +601,7 @@ mmc_status mmc_serve_create(mmc_heap* heap, uint32_t slots, uint32_t max_chunks,
     st = cuda_check(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     if(st == MMC_OK)
     {
-        mmc_status e = enqueue_tick(s, true);
+        mmc_status e = enqueue_tick(s);
         st = cuda_check(cudaStreamEndCapture(s->stream, &s->graph), "end capture");
         if(st == MMC_OK)
             st = e;
