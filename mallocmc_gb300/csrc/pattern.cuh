@@ -105,3 +105,57 @@ __device__ __forceinline__ void thread_pattern(char* ptr, uint32_t bytes, uint64
         }
     }
 }
+
+/* The verify workload's payload: n copies of the 32-bit word `value` from p
+ * (4-byte aligned) on, written, or read back and the words that differ counted,
+ * by one thread. Whole 32-byte sectors per access where the block has them: its
+ * lanes' accesses fall in as many sectors as there are lanes, and word by word
+ * each cost a request of its own (a million blocks of 8 to 600 bytes, one
+ * kernel to allocate and one to verify and free: 968 -> 370 us). */
+__device__ __forceinline__ void fill_words(uint32_t* p, uint32_t n, uint32_t value)
+{
+    const uint64_t a = __cvta_generic_to_global(p);
+    const uint32_t head = min(static_cast<uint32_t>(0u - a) >> 2 & 7u, n); /* words before the first whole sector */
+    const uint32_t sectors = (n - head) / 8u;
+    const uint64_t two = static_cast<uint64_t>(value) << 32 | value;
+    for(uint32_t i = 0; i < head; ++i)
+        p[i] = value;
+#pragma unroll 4
+    for(uint32_t i = 0; i < sectors; ++i)
+        asm volatile("st.global.v4.u64 [%0], {%1, %1, %1, %1};" ::"l"(a + 4u * head + 32u * i), "l"(two) : "memory");
+    for(uint32_t i = head + 8u * sectors; i < n; ++i)
+        p[i] = value;
+}
+
+__device__ __forceinline__ uint32_t wrong_words(const uint32_t* p, uint32_t n, uint32_t value)
+{
+    const uint64_t a = __cvta_generic_to_global(p);
+    const uint32_t head = min(static_cast<uint32_t>(0u - a) >> 2 & 7u, n);
+    const uint32_t sectors = (n - head) / 8u;
+    const uint64_t two = static_cast<uint64_t>(value) << 32 | value;
+    uint32_t bad = 0u;
+    for(uint32_t i = 0; i < head; ++i)
+        bad += p[i] != value;
+#pragma unroll 1
+    for(uint32_t i = 0; i < sectors; i += 4u)
+    {
+        Units2 v[4];
+#pragma unroll
+        for(uint32_t j = 0; j < 4u; ++j)
+            v[j] = ld_units2(a + 4u * head + 32u * (i + j), i + j, sectors);
+#pragma unroll
+        for(uint32_t j = 0; j < 4u; ++j)
+        {
+            if(i + j >= sectors)
+                continue;
+            const uint64_t d[4] = {v[j].w[0] ^ two, v[j].w[1] ^ two, v[j].w[2] ^ two, v[j].w[3] ^ two};
+            if((d[0] | d[1] | d[2] | d[3]) != 0ull)
+#pragma unroll
+                for(uint32_t k = 0; k < 4u; ++k)
+                    bad += (static_cast<uint32_t>(d[k]) != 0u) + (static_cast<uint32_t>(d[k] >> 32) != 0u);
+        }
+    }
+    for(uint32_t i = head + 8u * sectors; i < n; ++i)
+        bad += p[i] != value;
+    return bad;
+}

@@ -468,7 +468,6 @@ __global__ void __launch_bounds__(1024) mmc_verify_kernel(mmc_device_handle h, u
     if(t >= nthreads)
         return;
     const uint32_t pattern = t ^ seed;
-    const uint32_t words = dv::apply_padding(h.dataAlignment, sizes[t]) / 4u;
     uint32_t* p = nullptr;
     if(ALLOC)
     {
@@ -479,22 +478,18 @@ __global__ void __launch_bounds__(1024) mmc_verify_kernel(mmc_device_handle h, u
             p = static_cast<uint32_t*>(dv::malloc<dv::SmallRequests<Ids>>(h, sizes[t]));
         offsets[t] = p ? static_cast<int64_t>(reinterpret_cast<char*>(p) - h.pages) : -1;
         if(p)
-            for(uint32_t i = 0; i < sizes[t] / 4u; ++i)
-                p[i] = pattern;
+            fill_words(p, sizes[t] / 4u, pattern);
     }
     else
     {
         const int64_t off = offsets[t];
         p = off >= 0 ? reinterpret_cast<uint32_t*>(h.pages + off) : nullptr;
     }
-    (void) words;
     if(FREE && p)
     {
-        unsigned long long bad = 0;
-        for(uint32_t i = 0; i < sizes[t] / 4u; ++i)
-            bad += (p[i] != pattern);
+        const uint32_t bad = wrong_words(p, sizes[t] / 4u, pattern);
         if(bad)
-            atomicAdd(errors, bad);
+            atomicAdd(errors, static_cast<unsigned long long>(bad));
         dv::free<Ids>(h, p);
     }
 }
