@@ -208,9 +208,15 @@ namespace mmc
             return r;
         }
         /* The lanes that run here together, as a value to keep: a bare
-         * activemask may be read again by the compiler where the lanes have
+         * activemask (and a ballot of a constant over it, which is the same
+         * value) may be read again by the compiler where the lanes have
          * parted, and barriers on what it then gives wait for one another. */
-        __device__ __forceinline__ u32 converged_lanes() { return __ballot_sync(__activemask(), true); }
+        __device__ __forceinline__ u32 converged_lanes()
+        {
+            u32 lane;
+            asm("mov.u32 %0, %%laneid;" : "=r"(lane));
+            return __reduce_or_sync(__activemask(), 1u << lane);
+        }
         __device__ __forceinline__ u32 umin(u32 a, u32 b) { return a < b ? a : b; }
         __device__ __forceinline__ u32 umax(u32 a, u32 b) { return a > b ? a : b; }
         __device__ __forceinline__ u32 divup(u32 a, u32 b) { return (a + b - 1u) / b; }
@@ -576,16 +582,17 @@ namespace mmc
          * the heap after its refill counting every walk, 0.9783 this way (the
          * reference's serial run: 0.9750).
          *
-         * The warp's walking lanes go step by step together: per step each
-         * moves to its next region if it has to and tries one page. Left to
-         * itself the compiler threads the jumps of the lanes that pass a page
-         * around those that try one, and they no longer meet (up to twice the
-         * instructions on the uniform stress). One attempt serves every page,
-         * and malloc has one call of all this: with an attempt for each kind
-         * of region, each with unrolled claim retries, and two call sites in
-         * malloc, a kernel that allocates had 100 to 180 KB of code, and
-         * instruction fetch was the first stall of the stress and batched
-         * kernels. */
+         * One attempt serves every page, and malloc has one call of all this:
+         * with an attempt for each kind of region, each with unrolled claim
+         * retries, and two call sites in malloc, a kernel that allocates had
+         * 100 to 180 KB of code, and instruction fetch was the first stall of
+         * the stress and batched kernels.
+         *
+         * The lanes of a warp do not wait for one another in here. Walking
+         * step by step together they took fewer instructions (4.99 against
+         * 5.8 ms on the uniform stress, 0.95 against 0.9 on smaller sizes),
+         * but a few launches in a hundred of a 16 to 256 byte stress did not
+         * end. */
         template<class Ids>
         __device__ __forceinline__ void* alloc_chunked_walk(const mmc_device_handle& h, u32 bytes, u32 minAllocation,
                                                             u32 maxchunksize, u32 start, u32 level)
@@ -611,9 +618,6 @@ namespace mmc
                 i = R;
             void* res = nullptr;
             bool go = true;
-            u32 am = 1u;
-            if constexpr(Ids::warpSize > 1u)
-                am = converged_lanes();
             do
             {
                 bool read = false;
@@ -694,14 +698,9 @@ namespace mmc
                     res = attempt_page<Ids>(h, page, before, bytes, minAllocation, maxchunksize);
                     go = res == nullptr;
                 }
-                if constexpr(Ids::warpSize > 1u)
-                {
-                    if(!__any_sync(am, go))
-                        break;
-                }
-                else if(!go)
-                    break;
-            } while(true);
+                /* (keeps the compiler from threading the next step's jumps) */
+                asm volatile("" ::: "memory");
+            } while(go);
             return res;
         }
 
@@ -851,9 +850,7 @@ namespace mmc
             bool served = false;
             if constexpr(Ids::warpSize > 1u)
             {
-                const u32 am = converged_lanes();
                 served = claim_same_size<Ids>(h, bytes, minAllocation, maxchunksize, global_start_page, fill0, cs0, res);
-                __syncwarp(am);
             }
             if(!served && fill0 < R * 3u / 4u)
             {
