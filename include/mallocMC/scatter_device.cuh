@@ -280,6 +280,15 @@ namespace mmc
             atomicOr(&fm[page >> 5], 1u << (page & 31u));
         }
 
+        /* Behind the free-page bitmap lies a second one, with the bits of the
+         * pages that are in no multi-page run: all that a chunk walk has to
+         * look at. A run clears its bits once it is marked (its asker's fence
+         * waits for that before the run is handed out), and its free sets
+         * them, with a fence, before the pages' chunk sizes go to 0: a bit may
+         * stay set on a run's page, never clear on another. */
+        __host__ __device__ __forceinline__ u32 freemap_words(u32 numpages) { return ((numpages / 32u + 4u) & ~3u) + 4u; }
+        __device__ __forceinline__ u32* walkmap(u32* fm, u32 numpages) { return fm + freemap_words(numpages); }
+
         /* set (free) or clear the bits of pages [first, first + n), one atomic per word */
         __device__ inline void freemap_range(u32* fm, u32 first, u32 n, bool free)
         {
@@ -564,9 +573,14 @@ namespace mmc
          * region is read whole (region_candidates) and only its usable pages
          * are tried, in the reference's order from the entry page: a walk that
          * crosses regions of full pages or of multi-page runs costs a few
-         * round trips per region instead of one or two per page. The region counters are looked at
-         * eight regions ahead, so a stretch of regions skipped as 3/4 full
-         * costs one round trip per eight. Alone on the heap every page gets
+         * round trips per region instead of one or two per page. The region
+         * counters are looked at eight regions ahead, so a stretch of regions
+         * skipped as 3/4 full costs one round trip and one step per eight;
+         * read with them, a word of the map of pages outside multi-page runs
+         * has both passes skip the regions that runs fill as well. (The 32 GiB fragmentation run's two
+         * waves up to its first NULL: 800 and 50 to 1140 ms a region at a
+         * time, 850 and 915 by the counters alone, 226 and 550 so; the whole
+         * run 2.2 to 3.4 s, now 1.3 s.) Alone on the heap every page gets
          * the reference's outcome, in the reference's order.
          *
          * The counters: the reference counts every failed walk, whatever size
@@ -579,7 +593,7 @@ namespace mmc
          * first pass (the second walks every region anyway, and would mark the
          * whole heap). The 32 GiB fragmentation run, whose multi-page requests
          * are served fast enough to fill the heap to its last page: 0.9713 of
-         * the heap after its refill counting every walk, 0.9783 this way (the
+         * the heap after its refill counting every walk, 0.978 this way (the
          * reference's serial run: 0.9750).
          *
          * One attempt serves every page, and malloc has one call of all this:
@@ -590,9 +604,8 @@ namespace mmc
          *
          * The lanes of a warp do not wait for one another in here. Walking
          * step by step together they took fewer instructions (4.99 against
-         * 5.8 ms on the uniform stress, 0.95 against 0.9 on smaller sizes),
-         * but a few launches in a hundred of a 16 to 256 byte stress did not
-         * end. */
+         * 5.8 ms on the uniform stress), but a few launches in a hundred of a
+         * 16 to 256 byte stress did not end. */
         template<class Ids>
         __device__ __forceinline__ void* alloc_chunked_walk(const mmc_device_handle& h, u32 bytes, u32 minAllocation,
                                                             u32 maxchunksize, u32 start, u32 level)
@@ -600,12 +613,14 @@ namespace mmc
             const u32 R = h.regionsize;
             const u32 numregions = h.numregions;
             const bool batched = (R % 4u) == 0u && R <= 32u;
+            const bool mapped = Ids::warpSize > 1u && batched && (R & (R - 1u)) == 0u; /* a region's bits lie in one word */
             const u32 rmask = R >= 32u ? 0xFFFFFFFFu : ((1u << R) - 1u);
             u32 region = start / R;
             const u32 s0 = start - region * R;
             u32 checklevel = R * 3u / 4u;
             u64 ahead = 0u; /* counters of the regions ahead, a byte each */
             u32 known = 1u; /* how many, with this one */
+            u32 edge = 0u; /* the page where the next access block begins, once it is needed */
             u32 left = 2u * numregions; /* regions to visit, in both passes, this one included */
             /* Visiting index i is page region * R + (s0 + i) % R. With masks, the
              * usable pages (todo) and the unformatted ones (zero) go by it;
@@ -636,18 +651,37 @@ namespace mmc
                     }
                     else
                         MMC_STAT(h, MMC_STAT_REGION_SKIP);
-                    if(++region == numregions)
-                        region = 0u;
-                    if(s0 == 0u && (region * R) % h.pagesperblock == 0u)
+                    if(edge == 0u)
+                        edge = (region * R / h.pagesperblock + 1u) * h.pagesperblock;
+                    /* with it, the regions behind it that are passed by their
+                     * counters, as far as those are known, up to the pass's end */
+                    u32 n = 1u;
+                    if(Ids::warpSize > 1u && checklevel <= 255u)
                     {
-                        const u32 access_block_id = region * R / h.pagesperblock;
-                        /* racy by design (Scatter.hpp:625-628) */
-                        if(access_block_id > ld_rlx(&h.state->firstfreeblock))
-                            st_rlx(&h.state->firstfreeblock, access_block_id);
+                        const u32 check = checklevel * 0x01010101u;
+                        const u64 rest = ahead >> 8;
+                        const u32 lo = ~__vcmpgeu4(static_cast<u32>(rest), check);
+                        const u32 hi = ~__vcmpgeu4(static_cast<u32>(rest >> 32), check);
+                        const u32 full = static_cast<u32>(lo != 0u ? __ffs(static_cast<int>(lo)) - 1
+                                                                    : 32 + ((__ffs(static_cast<int>(hi)) - 1) & 31)) / 8u;
+                        n += umin(umin(full, known - 1u), (left > numregions ? left - numregions : left) - 1u);
                     }
-                    ahead >>= 8;
-                    --known;
-                    if(--left == numregions)
+                    region += n;
+                    if(region == numregions)
+                        region = 0u;
+                    if(region * R >= edge || region == 0u)
+                    {
+                        /* racy by design (Scatter.hpp:625-628) */
+                        const u32 access_block_id = region * R / h.pagesperblock;
+                        if(s0 == 0u && (region * R == access_block_id * h.pagesperblock || h.pagesperblock % R == 0u)
+                           && access_block_id > ld_rlx(&h.state->firstfreeblock))
+                            st_rlx(&h.state->firstfreeblock, access_block_id);
+                        edge = (access_block_id + 1u) * h.pagesperblock;
+                    }
+                    ahead = n < 8u ? ahead >> (8u * n) : 0u;
+                    known -= n;
+                    left -= n;
+                    if(left == numregions)
                     {
                         /* the second pass walks every region */
                         checklevel = R + 1u;
@@ -661,7 +695,16 @@ namespace mmc
 #pragma unroll
                         for(u32 k = 0; k < 8u; ++k)
                             if(k < known)
-                                ahead |= static_cast<u64>(umin(ld_rlx(&h.regions[region + k]), 255u)) << (8u * k);
+                            {
+                                u32 full = umin(ld_rlx(&h.regions[region + k]), 255u);
+                                if(mapped)
+                                {
+                                    const u32 first = (region + k) * R;
+                                    const u32 look = ld_rlx(&walkmap(h.freemap, h.numpages)[first >> 5]) >> (first & 31u);
+                                    full = (look & rmask) != 0u ? full : 255u;
+                                }
+                                ahead |= static_cast<u64>(full) << (8u * k);
+                            }
                     }
                     /* the counter as it was looked at, up to eight regions ago: of
                      * several walks that fail here together one raises it */
@@ -1108,6 +1151,7 @@ namespace mmc
                 }
             }
             freemap_range(c.freemap, startpage, pages, false);
+            freemap_range(walkmap(c.freemap, c.numpages), startpage, pages, false);
             asm volatile("fence.acq_rel.gpu;" ::: "memory");
             return true;
         }
@@ -1804,6 +1848,10 @@ namespace mmc
                     }
                     if(!__any_sync(kFull, lost != 0u))
                     {
+                        u32* wm = walkmap(c.freemap, c.numpages);
+                        for(u32 w = (first >> 5) + lane; 32u * w < first + pages; w += 32u)
+                            atomicAnd(&wm[w], ~word_span(w, first, first + pages));
+                        __threadfence();
                         if(lane == static_cast<u32>(j))
                         {
                             res = c.pages + static_cast<u64>(first) * c.pagesize;
@@ -1842,6 +1890,7 @@ namespace mmc
             const u32 end = umin(page + pages, h.numpages);
             for(u32 p = page; p < end; ++p)
                 page_init(h, p);
+            freemap_range(walkmap(h.freemap, h.numpages), page, end - page, true);
             __threadfence();
             for(u32 p = page; p < end; ++p)
                 atomicCAS(&h.chunksize[p], bytes, 0u);
@@ -1871,6 +1920,8 @@ namespace mmc
                 for(u32 p = first; p < end; ++p, tail += c.pagesize)
                     for(u32 w = rank; w < masks; w += g)
                         st_rlx(reinterpret_cast<u32*>(tail) + w, 0u);
+                for(u32 w = (first >> 5) + rank; 32u * w < end; w += g)
+                    atomicOr(&walkmap(c.freemap, c.numpages)[w], word_span(w, first, end));
                 __threadfence();
                 __syncwarp(am);
                 u32 old = tag;

@@ -114,7 +114,8 @@ typedef struct mmc_device_handle
     uint32_t* regions;   /* per-region fill counters */
     uint32_t* freemap;   /* free-page bitmap: bit (i & 31) of word i >> 5 is set while page i
                             has chunk size 0 (heap-owned, outside the pool; read by the
-                            concurrent multi-page search) */
+                            concurrent multi-page search); behind it, alike, the map of
+                            the pages outside multi-page runs, read by chunk walks */
     uint32_t numpages;
     uint32_t numregions;
     uint32_t accessblocks;

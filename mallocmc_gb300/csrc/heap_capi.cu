@@ -105,9 +105,10 @@ __global__ void mmc_init_kernel(mmc_device_handle h, uint32_t freemap_words)
 {
     /* every page starts free: its bit set; bits past numpages stay clear, so
      * the multi-page search sees them (and page numpages) as used */
+    const uint32_t half = mmc::dev::freemap_words(h.numpages); /* then the map of the walks, alike */
     for(uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < freemap_words; w += gridDim.x * blockDim.x)
     {
-        const uint32_t first = w * 32u;
+        const uint32_t first = (w < half ? w : w - half) * 32u;
         h.freemap[w] = first >= h.numpages ? 0u
                                            : (h.numpages - first >= 32u ? 0xFFFFFFFFu
                                                                          : (1u << (h.numpages - first)) - 1u);
@@ -483,7 +484,7 @@ namespace
     /* words of the free-page bitmap: one bit per page and a clear bit for page
      * numpages, rounded up to whole 16-byte groups (the search reads four
      * words at a time) and one spare group */
-    size_t freemap_words_for(uint32_t numpages) { return ((static_cast<size_t>(numpages) / 32u + 1u + 3u) & ~size_t{3}) + 4u; }
+    size_t freemap_words_for(uint32_t numpages) { return 2u * mmc::dev::freemap_words(numpages); }
 
     mmc_status init_heap(mmc_heap* h, cudaStream_t s)
     {
