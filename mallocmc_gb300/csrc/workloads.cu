@@ -240,11 +240,10 @@ __device__ __noinline__ void* malloc_large(const mmc_device_handle h, uint32_t b
  * about 6 % faster on GB300 than the one without the bound.
  *
  * A warp whose requests all fit a page, the usual one, runs its rounds without
- * the multi-page path: with the call of it in the loop ptxas spilled 172 bytes
- * at that bound (5.92 against 4.97 ms on the uniform stress), and with both
- * loops inlined 252 (5.52 ms). It looks the
- * size table through first, when there is one, 200 bytes a thread of the
- * benchmark's. */
+ * the multi-page path: with the call of it in the loop ptxas spilled 268 bytes
+ * at that bound (6.95 against 5.80 ms on the uniform stress), and with both
+ * loops inlined 348 (6.50 ms). It looks the size table through first, when
+ * there is one, 200 bytes a thread of the benchmark's. */
 template<uint32_t PATTERN, class Ids>
 __global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h, mmc_stress_params p,
                                                          const uint16_t* sizes, unsigned long long* stats)
