@@ -219,6 +219,57 @@ namespace
             h.free(c);
     }
 
+    using ChurnAllocator = PolicyAllocator<Sc, Xm, Ab, Sh>;
+
+    /* Threads that allocate, write, read back and free on schedules of their
+     * own: a thread sits rounds out and keeps its block for some, so the lanes
+     * of a warp come to malloc and free in changing groups. A pointer is used
+     * only if its block lies inside the pool. counts: blocks served, NULLs,
+     * pointers that are unaligned or outside the pool, words read back wrong. */
+    __global__ void churnKernel(ChurnAllocator::AllocatorHandle h, unsigned rounds, unsigned lo, unsigned hi,
+                                const char* pool, size_t pool_size, unsigned long long* counts)
+    {
+        const Acc acc{};
+        const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
+        unsigned* held = nullptr;
+        unsigned words = 0u, tag = 0u;
+        for(unsigned r = 0; r <= rounds; ++r)
+        {
+            unsigned x = id * 2654435761u + r * 0x9E3779B9u;
+            x = (x ^ (x >> 16)) * 0x85EBCA6Bu;
+            x ^= x >> 13;
+            if(held == nullptr && (x & 3u) != 0u && r < rounds)
+            {
+                const unsigned bytes = lo + (x >> 8) % (hi - lo + 1u);
+                char* p = static_cast<char*>(h.malloc(acc, bytes));
+                const size_t offset = static_cast<size_t>(p - pool);
+                if(p == nullptr)
+                    atomicAdd(&counts[1], 1ull);
+                else if(offset >= pool_size || bytes > pool_size - offset || offset % ShrinkConfig::dataAlignment != 0u)
+                    atomicAdd(&counts[2], 1ull);
+                else
+                {
+                    atomicAdd(&counts[0], 1ull);
+                    held = reinterpret_cast<unsigned*>(p);
+                    words = bytes / 4u;
+                    tag = x;
+                    for(unsigned i = 0; i < words; ++i)
+                        held[i] = tag + i;
+                }
+            }
+            else if(held != nullptr && ((x & 4u) != 0u || r == rounds))
+            {
+                unsigned wrong = 0u;
+                for(unsigned i = 0; i < words; ++i)
+                    wrong += held[i] != tag + i ? 1u : 0u;
+                if(wrong != 0u)
+                    atomicAdd(&counts[3], static_cast<unsigned long long>(wrong));
+                h.free(acc, held);
+                held = nullptr;
+            }
+        }
+    }
+
     int report(const std::exception& e)
     {
         std::fprintf(stderr, "mmcx: %s\n", e.what());
@@ -346,6 +397,34 @@ int mmcx_oldmalloc(int device, int length, unsigned long long* sum, unsigned lon
         cudaFree(d_fail);
         cudaFree(d_sums);
         return e == cudaSuccess ? 0 : 2;
+    }
+    catch(const std::exception& e)
+    {
+        return report(e);
+    }
+}
+
+/* Threads on schedules of their own (churnKernel) over a 1 GiB heap: counts[4]
+ * = {blocks served, NULLs, bad pointers, wrong words}, *flags the heap's device
+ * error bits. 3: the launch was refused. */
+int mmcx_churn(int device, unsigned blocks, unsigned threads, unsigned rounds, unsigned lo, unsigned hi,
+               unsigned long long* counts, unsigned* flags)
+{
+    try
+    {
+        cudaSetDevice(device);
+        ChurnAllocator alloc(device, nullptr, 1U * 1024U * 1024U * 1024U);
+        const auto pool = alloc.getHeapLocations().at(0);
+        unsigned long long* d_counts = nullptr;
+        cudaMalloc(&d_counts, 4 * sizeof(unsigned long long));
+        cudaMemset(d_counts, 0, 4 * sizeof(unsigned long long));
+        churnKernel<<<blocks, threads>>>(alloc.getAllocatorHandle(), rounds, lo, hi, static_cast<const char*>(pool.p),
+                                         pool.size, d_counts);
+        const bool refused = cudaGetLastError() != cudaSuccess;
+        cudaMemcpy(counts, d_counts, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
+        *flags = alloc.errorFlags();
+        cudaFree(d_counts);
+        return refused ? 3 : (cudaDeviceSynchronize() == cudaSuccess ? 0 : 2);
     }
     catch(const std::exception& e)
     {

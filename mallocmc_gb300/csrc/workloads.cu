@@ -25,6 +25,20 @@ namespace
         z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
         return z ^ (z >> 31);
     }
+
+    /* The lanes of this warp that have a thread, of those whose index is below
+     * n (the caller's is) in a one-dimensional launch: known by arithmetic, for
+     * warp-wide operations at the top of a kernel. */
+    __device__ __forceinline__ uint32_t warp_lanes()
+    {
+        const uint32_t here = blockDim.x - (threadIdx.x & ~31u);
+        return here >= 32u ? 0xFFFFFFFFu : (1u << here) - 1u;
+    }
+    __device__ __forceinline__ uint32_t warp_lanes(uint32_t n)
+    {
+        const uint32_t below = n - (blockIdx.x * blockDim.x + (threadIdx.x & ~31u));
+        return warp_lanes() & (below >= 32u ? 0xFFFFFFFFu : (1u << below) - 1u);
+    }
 } // namespace
 
 /* One thread, SerialIds: the reference's CPU-serial semantics. */
@@ -260,7 +274,7 @@ __global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h,
             most = max(most, static_cast<uint32_t>(mine[static_cast<uint64_t>(r) * nthreads]));
     }
     StressCounts n{};
-    if(__any_sync(__activemask(), dv::apply_padding(Ids::alignment(h), most) > h.pagesize))
+    if(__any_sync(warp_lanes(), dv::apply_padding(Ids::alignment(h), most) > h.pagesize))
         n = stress_rounds_large<PATTERN, Ids>(h, p, sizes, pieces);
     else
         stress_rounds<PATTERN, dv::SmallRequests<Ids>>(h, p, sizes, pieces, n);
@@ -471,7 +485,7 @@ __global__ void __launch_bounds__(1024) mmc_verify_kernel(mmc_device_handle h, u
     if(ALLOC)
     {
         /* warps whose requests all fit a page keep clear of the multi-page path (see the stress kernel) */
-        if(__any_sync(__activemask(), dv::apply_padding(Ids::alignment(h), sizes[t]) > h.pagesize))
+        if(__any_sync(warp_lanes(nthreads), dv::apply_padding(Ids::alignment(h), sizes[t]) > h.pagesize))
             p = static_cast<uint32_t*>(malloc_large<Ids>(h, sizes[t]));
         else
             p = static_cast<uint32_t*>(dv::malloc<dv::SmallRequests<Ids>>(h, sizes[t]));
