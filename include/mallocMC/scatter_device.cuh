@@ -1372,11 +1372,6 @@ namespace mmc
             return res;
         }
 
-        __device__ __forceinline__ void set_page_timeout(const PageScan& c)
-        {
-            atomicOr(&c.state->error_flags, MMC_DEVERR_TIMEOUT);
-        }
-
         /* ---------------------------- multi-page requests of whole warps
          * Every concurrent search of the lock-free form above settles on the
          * same run, the topmost that fits, and one of them gets it per round
@@ -1404,8 +1399,8 @@ namespace mmc
         constexpr u32 kPageGone = 0xC0000000u; /* ring word of a request given up */
         constexpr u32 kPageAnswer = 0x40000000u; /* ring word of an answer: | first page */
         constexpr u32 kPageNone = 0x3FFFFFFFu; /* answer's page when there is no run */
+        constexpr u32 kPageSearch = 0x7FFFFFFFu; /* "use the lock-free search", not in the ring */
         constexpr u32 kServiceMaxPages = 1024u; /* 32 claims per lane, remembered in one word */
-        constexpr u32 kServiceSlots = 8u; /* requests per lane in a batch */
         constexpr u32 kServiceRetries = 4u; /* runs lost to chunk pages before the lock-free search is used */
 
         __device__ __forceinline__ mmc_page_service* page_service(mmc_heap_state* state)
@@ -1455,62 +1450,142 @@ namespace mmc
             return n == 32u ? 0xFFFFFFFFu : ((1u << n) - 1u) << (lo & 31u);
         }
 
-        /* One pass of a batch's requests over the windows from page `top` down
-         * to page `low` (both included), by a whole warp holding the lock.
-         * req[s] holds a request's pages, 0, or a served request's
-         * kPageAsk | first page. With `hinting`, hint receives the highest page
-         * from which a later search could still find a multi-page run. */
-        __device__ __forceinline__ void page_service_pass(const PageScan& c, u32 (&req)[kServiceSlots], u32 top, u32 low,
-                                                          bool hinting, u32& hint)
+        /* A kernel that calls malloc has the registers of its deepest call path,
+         * taken or not. In one function the service took 103 to 124: a user's
+         * kernel had two blocks of 256 threads per SM for four, and blocks of
+         * 1024 threads were refused. So its steps are functions of their own (17
+         * to 38 registers), called one after another from create, and what
+         * lasts longer than a step lies in the kernel's stack frame (volatile:
+         * read where it is used). malloc and free in a user's loop take 56
+         * registers so, as without the service; with the steps called from a
+         * function between them, 64 to 70. In a batch, a lane's word k has the
+         * pages of requests 64 k + lane and 64 k + 32 + lane in its halves, 0
+         * for none or placed. */
+        constexpr u32 kServiceWords = 4u;
+        constexpr u32 kServiceSlots = 2u * kServiceWords;
+        constexpr u32 kServiceBatch = 32u * kServiceSlots;
+        struct PageCall
         {
+            PageScan c;
+            /* the asking lane's */
+            u32 bytes;
+            u32 stage;
+            u32 ticket;
+            u32 polls;
+            u32 run; /* first page of the run found, kPageNone: none */
+            /* the batch it serves */
+            u32 head;
+            u32 taken;
+            u32 asked; /* which of the lane's words get an answer */
+            u32 left; /* how many of them have no run yet */
+            u32 entry; /* the hint as the batch found it */
+            u32 w[kServiceWords];
+            u32 page[kServiceSlots]; /* first pages of those placed */
+        };
+        /* A request that finds no run, or is served, is over; one that is too
+         * large, or lost its runs to others, takes the lock-free search. */
+        enum PageStage : u32
+        {
+            kAsks,
+            kTicket, /* has a ticket, its word is not written yet */
+            kWaits,
+            kAnswered,
+            kSearches,
+            kOver
+        };
+
+        /* this lane's largest request of at most `fit` pages, 0: none */
+        __device__ __forceinline__ u32 largest_request(const volatile PageCall& r, u32 fit)
+        {
+            const u32 f = umin(fit, 0xFFFFu);
+            u32 most = 0u;
+#pragma unroll
+            for(u32 k = 0; k < kServiceWords; ++k)
+            {
+                const u32 v = r.w[k], lo = v & 0xFFFFu, hi = v >> 16;
+                most = umax(most, umax(lo <= f ? lo : 0u, hi <= f ? hi : 0u));
+            }
+            return most;
+        }
+
+        /* one of this lane's requests of n pages gets its first page */
+        __device__ __forceinline__ void place_request(volatile PageCall& r, u32 n, u32 page)
+        {
+            bool placed = false;
+#pragma unroll 1
+            for(u32 s = 0; !placed; ++s)
+            {
+                const u32 v = r.w[s / 2u], shift = 16u * (s & 1u);
+                placed = ((v >> shift) & 0xFFFFu) == n;
+                if(placed)
+                {
+                    r.w[s / 2u] = v & ~(0xFFFFu << shift);
+                    r.page[s] = page;
+                }
+            }
+            r.left = r.left - 1u;
+        }
+
+        /* the topmost run of n set bits of x, as the position of its lowest bit (there is one) */
+        __device__ __forceinline__ u32 topmost_run(u32 x, u32 n)
+        {
+            for(u32 got = 1u; got < n && x != 0u;)
+            {
+                const u32 d = umin(got, n - got);
+                x &= x >> d;
+                got += d;
+            }
+            return 31u - static_cast<u32>(__clz(static_cast<int>(x)));
+        }
+
+        /* One pass of a batch's requests over the windows from page `top` down
+         * to page `low` (both included), by a whole warp holding the lock. Returns
+         * the highest page from which a later search could still find a
+         * multi-page run. */
+        __device__ __noinline__ inline u32 page_service_pass(volatile PageCall* call, u32 top, u32 low)
+        {
+            volatile PageCall& req = *call;
+            u32* const freemap = req.c.freemap;
             constexpr u32 kFull = 0xFFFFFFFFu;
             const u32 lane = GpuIds::laneid();
-            const u32 wtop = top >> 10, wlow = low >> 10;
-            const u32 words = c.numpages / 32u + 1u;
+            u32 hint = top;
             u32 carry = 0u; /* free pages right above the window */
             bool open = true; /* no usable run was left above */
+            bool at_zero = false; /* a run was placed at page 0 */
+            u32 w = top >> 10;
             u32 ahead[4];
 #pragma unroll
             for(u32 k = 0; k < 4u; ++k)
-                ahead[k] = (wtop >= k && 32u * (wtop - k) + lane < words) ? ld_rlx(&c.freemap[32u * (wtop - k) + lane]) : 0u;
-            for(u32 w = wtop;; --w)
+                ahead[k] = (w >= k && 32u * (w - k) + lane <= req.c.numpages / 32u) ? ld_rlx(&freemap[32u * (w - k) + lane]) : 0u;
+            for(;; --w)
             {
-                u32 x = ahead[0];
+                u32 x = ahead[0] & word_span(32u * w + lane, low, top + 1u);
                 ahead[0] = ahead[1];
                 ahead[1] = ahead[2];
                 ahead[2] = ahead[3];
-                ahead[3] = w >= 4u ? ld_rlx(&c.freemap[32u * (w - 4u) + lane]) : 0u;
-                MMC_STAT_ADD(c, MMC_STAT_PAGE_SCAN, 32u);
-                x &= word_span(32u * w + lane, low, top + 1u);
-                const u32 base = 1024u * w;
-                const u32 any = __ballot_sync(kFull, x != 0u);
-                u32 pending = 0u;
-                if(any == 0u)
+                ahead[3] = w >= 4u ? ld_rlx(&freemap[32u * (w - 4u) + lane]) : 0u;
+                MMC_STAT_ADD(req.c, MMC_STAT_PAGE_SCAN, 32u);
+                if(__ballot_sync(kFull, x != 0u) == 0u)
                     carry = 0u;
                 else
                 {
                     for(;;)
                     {
                         const u32 t = static_cast<u32>(__clz(static_cast<int>(~x)));
-                        const u32 b = x == kFull ? 32u : static_cast<u32>(__ffs(static_cast<int>(~x))) - 1u;
                         const u32 notfull = __ballot_sync(kFull, x != kFull);
                         /* free pages right above this lane's word */
-                        const u32 higher = lane == 31u ? 0u : notfull >> (lane + 1u);
-                        const u32 j = lane + static_cast<u32>(__ffs(static_cast<int>(higher))); /* lowest of them */
-                        const u32 bj = __shfl_sync(kFull, b, static_cast<int>(j & 31u));
-                        const u32 above = higher == 0u ? 32u * (31u - lane) + carry : 32u * (j - lane - 1u) + bj;
+                        u32 above;
+                        {
+                            const u32 b = x == kFull ? 32u : static_cast<u32>(__ffs(static_cast<int>(~x))) - 1u;
+                            const u32 higher = lane == 31u ? 0u : notfull >> (lane + 1u);
+                            const u32 j = lane + static_cast<u32>(__ffs(static_cast<int>(higher))); /* lowest of them */
+                            const u32 bj = __shfl_sync(kFull, b, static_cast<int>(j & 31u));
+                            above = higher == 0u ? 32u * (31u - lane) + carry : 32u * (j - lane - 1u) + bj;
+                        }
                         const u32 len = longest_run(x);
                         const u32 fit = __reduce_max_sync(kFull, umax(x != 0u ? above + t : 0u, len));
                         /* the largest waiting request that fits */
-                        u32 mine = 0u;
-                        pending = 0u;
-#pragma unroll
-                        for(u32 s = 0; s < kServiceSlots; ++s)
-                        {
-                            const u32 v = req[s];
-                            pending |= (v != 0u && v < kPageAsk) ? 1u : 0u;
-                            mine = (v <= fit && v > mine) ? v : mine;
-                        }
+                        const u32 mine = largest_request(req, fit);
                         const u32 n = __reduce_max_sync(kFull, mine);
                         if(n == 0u)
                         {
@@ -1521,9 +1596,9 @@ namespace mmc
                                 open = false;
                                 const u32 hl = 31u - static_cast<u32>(__clz(static_cast<int>(__ballot_sync(kFull, x != 0u))));
                                 const u32 th = 31u - static_cast<u32>(__clz(static_cast<int>(__shfl_sync(kFull, x, static_cast<int>(hl)))));
-                                if(hinting)
-                                    hint = base + 32u * hl + th + (32u * hl + th == 1023u ? carry : 0u);
+                                hint = 1024u * w + 32u * hl + th + (32u * hl + th == 1023u ? carry : 0u);
                             }
+                            const u32 b = x == kFull ? 32u : static_cast<u32>(__ffs(static_cast<int>(~x))) - 1u;
                             const u32 l = static_cast<u32>(__ffs(static_cast<int>(notfull))) - 1u;
                             const u32 bl = __shfl_sync(kFull, b, static_cast<int>(l & 31u));
                             carry = notfull == 0u ? 1024u + carry : 32u * l + bl;
@@ -1532,362 +1607,380 @@ namespace mmc
                         /* its run: the topmost one */
                         const bool crossing = x != 0u && above + t >= n;
                         const u32 can = __ballot_sync(kFull, crossing || len >= n);
-                        const u32 src = 31u - static_cast<u32>(__clz(static_cast<int>(can)));
-                        u32 q = base + 32u * lane;
+                        u32 q = 1024u * w + 32u * lane;
                         if(crossing)
                             q += 32u + above - n;
-                        else
-                        {
-                            u32 y = x;
-                            for(u32 got = 1u; got < n && y != 0u;)
-                            {
-                                const u32 d = umin(got, n - got);
-                                y &= y >> d;
-                                got += d;
-                            }
-                            q += 31u - static_cast<u32>(__clz(static_cast<int>(y)));
-                        }
-                        q = __shfl_sync(kFull, q, static_cast<int>(src));
+                        else if(len >= n)
+                            q += topmost_run(x, n);
+                        q = __shfl_sync(kFull, q, 31 - __clz(static_cast<int>(can)));
+                        at_zero = at_zero || q == 0u;
                         const u32 used = word_span(32u * w + lane, q, q + n);
                         if(used != 0u)
                         {
                             x &= ~used;
-                            atomicAnd(&c.freemap[32u * w + lane], ~used);
+                            atomicAnd(&freemap[32u * w + lane], ~used);
                         }
-                        if(q + n > base + 1024u)
+                        if(q + n > 1024u * w + 1024u)
                         {
                             /* the part above the window */
-                            const u32 end = (q + n - 1u) >> 5;
-                            for(u32 ww = umax(32u * w + 32u, q >> 5) + lane; ww <= end; ww += 32u)
-                                atomicAnd(&c.freemap[ww], ~word_span(ww, q, q + n));
-                            carry = 0u;
+                            for(u32 ww = umax(32u * w + 32u, q >> 5) + lane; ww <= (q + n - 1u) >> 5; ww += 32u)
+                                atomicAnd(&freemap[ww], ~word_span(ww, q, q + n));
                         }
-                        else if(q + n == base + 1024u)
+                        if(q + n >= 1024u * w + 1024u)
                             carry = 0u; /* the pages above, if free, no longer join this window's */
-                        const u32 who = static_cast<u32>(__ffs(static_cast<int>(__ballot_sync(kFull, mine == n)))) - 1u;
-                        bool given = lane != who;
-#pragma unroll
-                        for(u32 s = 0; s < kServiceSlots; ++s)
-                            if(!given && req[s] == n)
-                            {
-                                req[s] = kPageAsk | q;
-                                given = true;
-                            }
+                        if(lane == static_cast<u32>(__ffs(static_cast<int>(__ballot_sync(kFull, mine == n)))) - 1u)
+                            place_request(req, n, q);
                     }
                 }
-                if(any == 0u)
-                {
-#pragma unroll
-                    for(u32 s = 0; s < kServiceSlots; ++s)
-                        pending |= (req[s] != 0u && req[s] < kPageAsk) ? 1u : 0u;
-                }
-                if(hinting && open)
-                    hint = base == 0u ? 0u : umin(base - 1u, top);
-                if(w == wlow || __ballot_sync(kFull, pending != 0u) == 0u)
+                if(open)
+                    hint = w == 0u ? 0u : umin(1024u * w - 1u, top);
+                if(w == low >> 10 || !__any_sync(kFull, req.left != 0u))
                     break;
             }
+            /* the reference stores a run's first page - 1, which wraps for a
+             * run at page 0 (Scatter.hpp:800-804); fixed mode stores 0 */
+            return at_zero && hint == 0u && req.c.reference_quirks ? 0xFFFFFFFFu : hint;
         }
 
-        /* Serve a batch (req[s]: pages or 0); answers replace the requests as
-         * kPageAsk | first page, what found no run stays. */
-        __device__ __forceinline__ void page_service_batch(const PageScan& c, u32 (&req)[kServiceSlots])
+        /* Pages (start - sum, start] all free, sum those of the batch's requests:
+         * it packs there. (A run at page 0 is left to the passes.) */
+        __device__ __noinline__ inline bool page_service_stretch(volatile PageCall* call, u32 sum)
         {
             constexpr u32 kFull = 0xFFFFFFFFu;
+            volatile PageCall& req = *call;
+            u32* const freemap = req.c.freemap;
             const u32 lane = GpuIds::laneid();
-            const u32 entry = ld_rlx(&c.state->firstFreePageBased);
-            /* the reference's wrapped hint: its searches visit no page */
-            if(entry == 0xFFFFFFFFu)
-                return;
-            const u32 start = umin(entry, c.numpages);
+            const u32 start = umin(req.entry, req.c.numpages);
+            if(sum >= start || start >= req.c.numpages)
+                return false;
+            const u32 low = start + 1u - sum;
+            for(u32 w0 = start >> 5;; w0 -= 128u)
+            {
+                bool ok = true;
+#pragma unroll
+                for(u32 k = 0; k < 4u; ++k)
+                {
+                    const u32 off = 32u * k + lane;
+                    const u32 w = w0 - off;
+                    const u32 need = off <= w0 ? word_span(w, low, start + 1u) : 0u;
+                    if(need != 0u)
+                        MMC_STAT_ADD(req.c, MMC_STAT_PAGE_SCAN, 32u);
+                    if(need != 0u)
+                        ok = ok && (ld_rlx(&freemap[w]) & need) == need;
+                }
+                if(!__all_sync(kFull, ok))
+                    return false;
+                if(w0 < 128u || 32u * (w0 - 127u) <= low)
+                    break;
+            }
+            for(u32 w = (low >> 5) + lane; w <= (start >> 5); w += 32u)
+                atomicAnd(&freemap[w], ~word_span(w, low, start + 1u));
             u32 mine = 0u;
 #pragma unroll
-            for(u32 s = 0; s < kServiceSlots; ++s)
-                mine += req[s];
-            const u32 sum = __reduce_add_sync(kFull, mine);
-            if(sum == 0u)
-                return;
-            /* pages (start - sum, start] all free: the batch packs there (a run at page 0 is left to the passes) */
-            if(sum < start && start < c.numpages)
+            for(u32 k = 0; k < kServiceWords; ++k)
             {
-                const u32 low = start + 1u - sum;
-                bool all = true;
-                for(u32 w0 = start >> 5; all; )
-                {
-                    bool ok = true;
-#pragma unroll
-                    for(u32 k = 0; k < 4u; ++k)
-                    {
-                        const u32 off = 32u * k + lane;
-                        const u32 w = w0 - off;
-                        const u32 need = off <= w0 ? word_span(w, low, start + 1u) : 0u;
-                        if(need != 0u)
-                            MMC_STAT_ADD(c, MMC_STAT_PAGE_SCAN, 32u);
-                        if(need != 0u)
-                            ok = ok && (ld_rlx(&c.freemap[w]) & need) == need;
-                    }
-                    all = __all_sync(kFull, ok);
-                    if(w0 < 128u || 32u * (w0 - 127u) <= low)
-                        break;
-                    w0 -= 128u;
-                }
-                if(all)
-                {
-                    for(u32 w = (low >> 5) + lane; w <= (start >> 5); w += 32u)
-                        atomicAnd(&c.freemap[w], ~word_span(w, low, start + 1u));
-                    u32 incl = mine;
-#pragma unroll
-                    for(u32 off = 1u; off < 32u; off <<= 1)
-                    {
-                        const u32 v = __shfl_up_sync(kFull, incl, off);
-                        if(lane >= off)
-                            incl += v;
-                    }
-                    u32 next = start + 1u - (incl - mine);
-#pragma unroll
-                    for(u32 s = 0; s < kServiceSlots; ++s)
-                        if(req[s] != 0u)
-                        {
-                            next -= req[s];
-                            req[s] = kPageAsk | next;
-                        }
-                    if(lane == 0u)
-                        atomicCAS(&c.state->firstFreePageBased, entry, low - 1u);
-                    return;
-                }
+                const u32 v = req.w[k];
+                mine += (v & 0xFFFFu) + (v >> 16);
             }
-            /* from the hint down, then what is left from the top down to it */
-            u32 hint = start;
-#pragma unroll 1
-            for(u32 leg = 0; leg < 2u; ++leg)
+            u32 incl = mine;
+#pragma unroll
+            for(u32 off = 1u; off < 32u; off <<= 1)
             {
-                page_service_pass(c, req, leg == 0u ? start : c.numpages, leg == 0u ? 0u : start, leg == 0u, hint);
-                bool waiting = false, at_zero = false;
-#pragma unroll
-                for(u32 s = 0; s < kServiceSlots; ++s)
-                {
-                    waiting = waiting || (req[s] != 0u && req[s] < kPageAsk);
-                    at_zero = at_zero || req[s] == kPageAsk;
-                }
-                if(leg == 0u)
-                {
-                    /* the reference stores a run's first page - 1, which wraps for a
-                     * run at page 0 (Scatter.hpp:800-804); fixed mode stores 0 */
-                    if(__any_sync(kFull, at_zero) && hint == 0u && c.reference_quirks)
-                        hint = 0xFFFFFFFFu;
-                    if(lane == 0u && hint != entry)
-                        atomicCAS(&c.state->firstFreePageBased, entry, hint);
-                }
-                if(!__any_sync(kFull, waiting))
-                    break;
+                const u32 v = __shfl_up_sync(kFull, incl, off);
+                if(lane >= off)
+                    incl += v;
             }
+            u32 next = start + 1u - (incl - mine);
+#pragma unroll
+            for(u32 k = 0; k < kServiceWords; ++k)
+            {
+                const u32 v = req.w[k];
+                next -= v & 0xFFFFu;
+                req.page[2u * k] = next;
+                next -= v >> 16;
+                req.page[2u * k + 1u] = next;
+                req.w[k] = 0u;
+            }
+            if(lane == 0u)
+                atomicCAS(&req.c.state->firstFreePageBased, +req.entry, low - 1u);
+            return true;
         }
 
-        /* Serve what waits in the ring, batch by batch; the caller's warp (whole) holds the lock. */
-        __device__ __noinline__ inline void page_service_run(const PageScan c)
+        /* The next batch of the ring into the call's frame: the pages its
+         * requests ask for, all told; 0 for an empty batch. A ticket drawn but
+         * not written yet (its lane is about to) ends it. */
+        __device__ __noinline__ inline u32 page_service_take(volatile PageCall* call)
         {
             constexpr u32 kFull = 0xFFFFFFFFu;
-            mmc_page_service* sv = page_service(c.state);
+            volatile PageCall& req = *call;
+            mmc_page_service* sv = page_service(req.c.state);
             const u32 lane = GpuIds::laneid();
-            u32 head = ld_rlx(&sv->head);
-            for(u32 round = 0; round < 64u; ++round)
+            const u32 head = req.head;
+            const u32 have = __shfl_sync(kFull, umin(ld_rlx(&sv->tail) - head, kServiceBatch), 0);
+            u32 taken = have;
+#pragma unroll 1
+            for(u32 k = 0; k < kServiceWords; k += 2u)
             {
-                const u32 count = umin(ld_rlx(&sv->tail) - head, 32u * kServiceSlots);
-                if(__shfl_sync(kFull, count, 0) == 0u)
-                    break;
-                const u32 have = __shfl_sync(kFull, count, 0);
-                u32 req[kServiceSlots];
-                u32 taken = have;
+                u32 v[4];
 #pragma unroll
-                for(u32 s = 0; s < kServiceSlots; ++s)
+                for(u32 j = 0; j < 4u; ++j)
                 {
-                    const u32 i = 32u * s + lane;
-                    req[s] = i < have ? ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]) : 0u;
+                    const u32 i = 64u * k + 32u * j + lane;
+                    v[j] = i < have ? ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]) : 0u;
                 }
-                /* a ticket drawn but not written yet (its lane is about to): the batch ends before it */
 #pragma unroll
-                for(u32 s = 0; s < kServiceSlots; ++s)
+                for(u32 j = 0; j < 4u; ++j)
                 {
-                    const u32 i = 32u * s + lane;
-                    for(u32 spin = 0; i < taken && (req[s] & kPageAsk) == 0u; ++spin)
+                    const u32 i = 64u * k + 32u * j + lane;
+#pragma unroll 1
+                    for(u32 spin = 0; i < taken && (v[j] & kPageAsk) == 0u; ++spin)
                     {
+                        v[j] = ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]);
                         if(spin == 64u)
                             taken = i;
-                        else
-                            req[s] = ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]);
                     }
+                    /* given up: kept as 0xFFFF until it is known whether the batch has it */
+                    v[j] = v[j] == kPageGone ? 0xFFFFu : v[j] & 0xFFFFu;
                 }
-                taken = __reduce_min_sync(kFull, taken);
-                if(taken == 0u)
-                    break;
-#pragma unroll
-                for(u32 s = 0; s < kServiceSlots; ++s)
-                {
-                    const u32 i = 32u * s + lane;
-                    if(i < taken && req[s] == kPageGone)
-                        st_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)], 0u);
-                    req[s] = (i < taken && req[s] != kPageGone) ? req[s] & ~kPageAsk : 0u;
-                }
-                u32 asked = 0u;
-#pragma unroll
-                for(u32 s = 0; s < kServiceSlots; ++s)
-                    asked |= req[s] != 0u ? 1u << s : 0u;
-                page_service_batch(c, req);
-                /* every lane's bit clears are performed before any answer is seen */
-                __threadfence();
-                __syncwarp();
-#pragma unroll
-                for(u32 s = 0; s < kServiceSlots; ++s)
-                    if((asked >> s) & 1u)
-                    {
-                        u32* word = &sv->ring[(head + 32u * s + lane) & (MMC_PAGE_RING - 1u)];
-                        st_rlx(word, kPageAnswer | ((req[s] & kPageAsk) != 0u ? req[s] & ~kPageAsk : kPageNone));
-                    }
-                head += taken;
-                if(lane == 0u)
-                    st_rlx(&sv->head, head);
+                req.w[k] = v[0] | v[1] << 16;
+                req.w[k + 1u] = v[2] | v[3] << 16;
             }
-            __threadfence();
-            __syncwarp();
-            if(lane == 0u)
-                st_rlx(&sv->lock, 0u);
+            taken = __reduce_min_sync(kFull, taken);
+            u32 asked = 0u, sum = 0u;
+#pragma unroll 1
+            for(u32 s = 0; s < kServiceSlots; ++s)
+            {
+                const u32 w = req.w[s / 2u], shift = 16u * (s & 1u);
+                const u32 n = (w >> shift) & 0xFFFFu, i = 32u * s + lane;
+                const bool in = i < taken && n != 0xFFFFu;
+                if(i < taken && n == 0xFFFFu)
+                    st_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)], 0u);
+                if(!in)
+                    req.w[s / 2u] = w & ~(0xFFFFu << shift);
+                asked |= in && n != 0u ? 1u << s : 0u;
+                sum += in ? n : 0u;
+            }
+            req.taken = taken;
+            req.asked = asked;
+            req.left = static_cast<u32>(__popc(asked));
+            return __reduce_add_sync(kFull, sum);
         }
 
-        /* Multi-page requests of a whole warp: `bytes` per lane, 0 for none. */
-        __device__ __noinline__ inline char* alloc_page_based_warp(const PageScan c, u32 bytes)
+        /* Answer the batch's requests (those placed have no pages left) and pass it. */
+        __device__ __noinline__ inline void page_service_answer(volatile PageCall* call)
+        {
+            volatile PageCall& req = *call;
+            mmc_page_service* sv = page_service(req.c.state);
+            const u32 lane = GpuIds::laneid();
+            const u32 head = req.head;
+            /* every lane's bit clears are performed before any answer is seen */
+            __threadfence();
+            __syncwarp();
+#pragma unroll 1
+            for(u32 m = req.asked; m != 0u; m &= m - 1u)
+            {
+                const u32 s = static_cast<u32>(__ffs(static_cast<int>(m))) - 1u;
+                const bool none = ((req.w[s / 2u] >> (16u * (s & 1u))) & 0xFFFFu) != 0u;
+                const u32 page = req.page[s];
+                st_rlx(&sv->ring[(head + 32u * s + lane) & (MMC_PAGE_RING - 1u)], kPageAnswer | (none ? +kPageNone : page));
+            }
+            req.head = head + req.taken;
+            if(lane == 0u)
+                st_rlx(&sv->head, head + req.taken);
+        }
+
+        /* The requests of a whole warp enter the ring: a ticket for each lane that asks. */
+        __device__ __noinline__ inline bool page_service_enter(volatile PageCall* call)
+        {
+            const u32 asking = __ballot_sync(0xFFFFFFFFu, call->stage == kAsks);
+            if(asking == 0u)
+                return false;
+            u32 ticket = 0u;
+            if(GpuIds::laneid() == 0u)
+                ticket = atomicAdd(&page_service(call->c.state)->tail, static_cast<u32>(__popc(asking)));
+            ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0) + static_cast<u32>(__popc(asking & lanemask_lt()));
+            if(call->stage == kAsks)
+                call->stage = kTicket; /* (its run is kPageNone; the others' may have runs already) */
+            call->ticket = ticket;
+            call->polls = 0u;
+            return true;
+        }
+
+        /* One look at the ring by a waiting warp: 0 when all its requests are
+         * answered, 1 to look again, 2 when it has taken the lock to serve. */
+        __device__ __noinline__ inline u32 page_service_poll(volatile PageCall* call)
         {
             constexpr u32 kFull = 0xFFFFFFFFu;
-            mmc_page_service* sv = page_service(c.state);
-            const u32 lane = GpuIds::laneid();
-            const u32 n = divup(bytes, c.pagesize);
-            bool want = n != 0u && n <= kServiceMaxPages;
-            bool search = n > kServiceMaxPages;
-            char* res = nullptr;
-            for(u32 round = 0;; ++round)
+            mmc_page_service* sv = page_service(call->c.state);
+            const u32 ticket = call->ticket;
+            u32* word = &sv->ring[ticket & (MMC_PAGE_RING - 1u)];
+            const u32 polls = call->polls;
+            const bool late = polls > MMC_MUTEX_MAX_SPINS;
+            u32 stage = call->stage;
+            if(stage == kTicket)
             {
-                const u32 asking = __ballot_sync(kFull, want);
-                if(asking == 0u)
-                    break;
-                if(round == kServiceRetries)
+                /* a ticket's word is its own once the ticket a whole ring before
+                 * it has been served and its answer read */
+                if(ticket - ld_rlx(&sv->head) < MMC_PAGE_RING && ld_rlx(word) == 0u)
                 {
-                    search = search || want;
-                    break;
+                    st_rlx(word, kPageAsk | divup(call->bytes, call->c.pagesize));
+                    stage = kWaits;
                 }
-                u32 ticket = 0u, served = 0u;
-                if(lane == 0u)
+                else if(late)
+                    stage = kAnswered;
+            }
+            else if(stage == kWaits)
+            {
+                const u32 v = ld_rlx(word);
+                if((v & kPageAsk) == 0u)
                 {
-                    served = ld_rlx(&sv->head);
-                    ticket = atomicAdd(&sv->tail, static_cast<u32>(__popc(asking)));
+                    call->run = v & kPageNone;
+                    st_rlx(word, 0u);
+                    stage = kAnswered;
                 }
-                ticket = __shfl_sync(kFull, ticket, 0) + static_cast<u32>(__popc(asking & lanemask_lt()));
-                u32* word = &sv->ring[ticket & (MMC_PAGE_RING - 1u)];
-                /* a ticket's word is its own once the ticket a whole ring
-                 * before it has been served (and, below, its answer read) */
-                bool turn = ticket - __shfl_sync(kFull, served, 0) < MMC_PAGE_RING;
-                bool written = false, waiting = want;
-                u32 q = kPageNone;
-                for(u32 it = 0;; ++it)
-                {
-                    if(waiting && !written)
-                    {
-                        if(!turn)
-                            turn = ticket - ld_rlx(&sv->head) < MMC_PAGE_RING;
-                        if(turn && ld_rlx(word) == 0u)
-                        {
-                            st_rlx(word, kPageAsk | n);
-                            written = true;
-                        }
-                        else if(it > MMC_MUTEX_MAX_SPINS)
-                        {
-                            set_page_timeout(c);
-                            waiting = false;
-                        }
-                    }
-                    else if(waiting)
-                    {
-                        const u32 v = ld_rlx(word);
-                        if((v & kPageAsk) == 0u)
-                        {
-                            q = v & kPageNone;
-                            st_rlx(word, 0u);
-                            waiting = false;
-                        }
-                        else if(it > MMC_MUTEX_MAX_SPINS && atomicCAS(word, v, kPageGone) == v)
-                        {
-                            set_page_timeout(c);
-                            waiting = false;
-                        }
-                    }
-                    if(!__any_sync(kFull, waiting))
-                        break;
-                    u32 mine = 0u;
-                    if(lane == 0u && ld_rlx(&sv->lock) == 0u)
-                        mine = atomicCAS(&sv->lock, 0u, 1u) == 0u ? 1u : 0u;
-                    if(__shfl_sync(kFull, mine, 0) != 0u)
-                    {
-                        __threadfence();
-                        page_service_run(c);
-                    }
-                    else if(it > 1u)
-                        __nanosleep(umin(64u << umin(it, 5u), 1024u));
-                }
-                /* answers are read: what the server did to the bitmap is performed before what follows */
+                else if(late && atomicCAS(word, v, kPageGone) == v)
+                    stage = kAnswered;
+            }
+            if(late)
+                atomicOr(&call->c.state->error_flags, MMC_DEVERR_TIMEOUT);
+            call->stage = stage;
+            call->polls = polls + 1u;
+            if(!__any_sync(kFull, stage == kTicket || stage == kWaits))
+            {
+                /* what the server did to the bitmap is performed before what follows */
                 __threadfence();
-                if(want && q == kPageNone)
+                return 0u;
+            }
+            u32 lock = 1u;
+            if(GpuIds::laneid() == 0u && ld_rlx(&sv->lock) == 0u)
+                lock = atomicCAS(&sv->lock, 0u, 1u);
+            if(__shfl_sync(kFull, lock, 0) == 0u)
+            {
+                __threadfence();
+                call->head = ld_rlx(&sv->head);
+                return 2u;
+            }
+            if(polls > 1u)
+                __nanosleep(umin(64u << umin(polls, 5u), 1024u));
+            return 1u;
+        }
+
+        /* Serve what waits, batch by batch; the warp (whole) holds the lock. */
+        __device__ __forceinline__ void page_service_run(volatile PageCall* call)
+        {
+#pragma unroll 1
+            for(volatile u32 batch = 0; batch < 64u; batch = batch + 1u)
+            {
+                const u32 sum = page_service_take(call);
+                if(call->taken == 0u)
+                    break;
+                call->entry = ld_rlx(&call->c.state->firstFreePageBased);
+                /* (from the reference's wrapped hint searches visit no page) */
+                if(sum != 0u && call->entry != 0xFFFFFFFFu && !page_service_stretch(call, sum))
                 {
-                    MMC_STAT(c, MMC_STAT_PAGE_BASED_FAIL);
-                    want = false;
+                    /* from the hint down, then what is left from the top down to it */
+                    const u32 hint = page_service_pass(call, umin(call->entry, call->c.numpages), 0u);
+                    if(GpuIds::laneid() == 0u && hint != call->entry)
+                        atomicCAS(&call->c.state->firstFreePageBased, +call->entry, hint);
+                    if(__any_sync(0xFFFFFFFFu, call->left != 0u))
+                        page_service_pass(call, call->c.numpages, umin(call->entry, call->c.numpages));
+                }
+                page_service_answer(call);
+            }
+
+            __threadfence();
+            __syncwarp();
+            if(GpuIds::laneid() == 0u)
+                st_rlx(&page_service(call->c.state)->lock, 0u);
+        }
+
+        /* Claim the run that lane j was answered, a whole warp: 32 pages per
+         * instruction. A run that is lost is given back, to be asked for again. */
+        __device__ __noinline__ inline void claim_run_warp(volatile PageCall* call, int j)
+        {
+            constexpr u32 kFull = 0xFFFFFFFFu;
+            volatile PageCall& req = *call;
+            u32* const chunksize = req.c.chunksize;
+            const u32 lane = GpuIds::laneid();
+            const u32 first = __shfl_sync(kFull, req.run, j);
+            const u32 tag = __shfl_sync(kFull, req.bytes, j);
+            const u32 pages = divup(tag, req.c.pagesize);
+            u32 got = 0u, lost = 0u;
+#pragma unroll 4
+            for(u32 i = 0; i < divup(pages, 32u); ++i)
+            {
+                const u32 off = 32u * i + lane;
+                const u32 old = off < pages ? atomicCAS(&chunksize[first + off], 0u, tag) : 0u;
+                got |= (off < pages && old == 0u ? 1u : 0u) << i;
+                lost |= old;
+            }
+            const bool mine = lane == static_cast<u32>(j);
+            if(!__any_sync(kFull, lost != 0u))
+            {
+                u32* wm = walkmap(req.c.freemap, req.c.numpages);
+                for(u32 w = (first >> 5) + lane; 32u * w < first + pages; w += 32u)
+                    atomicAnd(&wm[w], ~word_span(w, first, first + pages));
+                __threadfence();
+                if(mine)
+                    req.stage = kOver;
+                return;
+            }
+            /* A page of the run went to a chunk format or a lock-free
+             * search: put the others back, as markpages does (each
+             * lost page's owner keeps its bit). */
+            MMC_STAT(req.c, MMC_STAT_PAGE_LOST);
+            if(mine)
+            {
+                req.run = kPageNone;
+                req.stage = kAsks;
+            }
+            u32 top = 0u;
+#pragma unroll 1
+            for(u32 m = got; m != 0u; m &= m - 1u)
+            {
+                const u32 page = first + 32u * (static_cast<u32>(__ffs(static_cast<int>(m))) - 1u) + lane;
+                if(atomicCAS(&chunksize[page], tag, 0u) == tag)
+                {
+                    freemap_set(req.c.freemap, page);
+                    top = page + 1u;
+                }
+            }
+            if(top != 0u)
+                atomicMax(&req.c.state->firstFreePageBased, top - 1u);
+        }
+
+        /* Multi-page requests of a whole warp, the call's bytes per lane, 0 for
+         * none: the first page of the lane's run, claimed, kPageNone, or
+         * kPageSearch where the lock-free search is to be used. */
+        __device__ __forceinline__ u32 alloc_page_based_warp(volatile PageCall* call)
+        {
+            {
+                const u32 n = divup(call->bytes, call->c.pagesize);
+                call->stage = n == 0u ? kOver : (n <= kServiceMaxPages ? kAsks : kSearches);
+                call->run = kPageNone;
+            }
+#pragma unroll 1
+            for(volatile u32 round = 0; round < kServiceRetries && page_service_enter(call); round = round + 1u)
+            {
+                for(u32 look = 1u; look != 0u;)
+                {
+                    look = page_service_poll(call);
+                    if(look == 2u)
+                        page_service_run(call);
+                }
+                if(call->stage == kAnswered && call->run == kPageNone)
+                {
+                    MMC_STAT(call->c, MMC_STAT_PAGE_BASED_FAIL);
+                    call->stage = kOver;
                 }
                 /* mark the runs, the warp together */
-                for(u32 todo = __ballot_sync(kFull, want); todo != 0u; todo &= todo - 1u)
-                {
-                    const int j = __ffs(static_cast<int>(todo)) - 1;
-                    const u32 first = __shfl_sync(kFull, q, j);
-                    const u32 pages = __shfl_sync(kFull, n, j);
-                    const u32 tag = __shfl_sync(kFull, bytes, j);
-                    u32 got = 0u, lost = 0u;
-#pragma unroll 4
-                    for(u32 i = 0; i < divup(pages, 32u); ++i)
-                    {
-                        const u32 off = 32u * i + lane;
-                        const u32 old = off < pages ? atomicCAS(&c.chunksize[first + off], 0u, tag) : 0u;
-                        got |= (off < pages && old == 0u ? 1u : 0u) << i;
-                        lost |= old;
-                    }
-                    if(!__any_sync(kFull, lost != 0u))
-                    {
-                        u32* wm = walkmap(c.freemap, c.numpages);
-                        for(u32 w = (first >> 5) + lane; 32u * w < first + pages; w += 32u)
-                            atomicAnd(&wm[w], ~word_span(w, first, first + pages));
-                        __threadfence();
-                        if(lane == static_cast<u32>(j))
-                        {
-                            res = c.pages + static_cast<u64>(first) * c.pagesize;
-                            want = false;
-                        }
-                        continue;
-                    }
-                    /* A page of the run went to a chunk format or a lock-free
-                     * search: put the others back, as markpages does (each
-                     * lost page's owner keeps its bit), and ask again. */
-                    MMC_STAT(c, MMC_STAT_PAGE_LOST);
-                    u32 top = 0u;
-                    for(u32 m = got; m != 0u; m &= m - 1u)
-                    {
-                        const u32 page = first + 32u * (static_cast<u32>(__ffs(static_cast<int>(m))) - 1u) + lane;
-                        if(atomicCAS(&c.chunksize[page], tag, 0u) == tag)
-                        {
-                            freemap_set(c.freemap, page);
-                            top = page + 1u;
-                        }
-                    }
-                    if(top != 0u)
-                        atomicMax(&c.state->firstFreePageBased, top - 1u);
-                }
+#pragma unroll 1
+                for(volatile u32 todo = __ballot_sync(0xFFFFFFFFu, call->stage == kAnswered); todo != 0u;
+                    todo = todo & (todo - 1u))
+                    claim_run_warp(call, __ffs(static_cast<int>(todo)) - 1);
                 __syncwarp();
             }
-            if(search)
-                res = alloc_page_based_concurrent(c, bytes);
-            return res;
+            return call->stage == kOver ? +call->run : +kPageSearch;
         }
 
         /* deallocPageBased, Scatter.hpp:874-886 (out of line, as the search) */
@@ -1912,9 +2005,10 @@ namespace mmc
          * took 202 us. The CASes have returned before the bits are set: a bit
          * set ahead of its CAS could be taken by the server, whose claim then
          * fails and leaves the page's bit clear for good. */
-        __device__ __noinline__ inline void dealloc_page_based_warp(const PageScan c, u32 masks, u32 am, u32 runs,
-                                                                    u32 page, u32 bytes)
+        __device__ __noinline__ inline void dealloc_page_based_warp(const volatile PageScan* context, u32 masks, u32 am,
+                                                                    u32 runs, u32 page, u32 bytes)
         {
+            const volatile PageScan& c = *context;
             const u32 g = static_cast<u32>(__popc(am));
             const u32 rank = static_cast<u32>(__popc(am & lanemask_lt()));
             for(u32 todo = runs; todo != 0u; todo &= todo - 1u)
@@ -1923,18 +2017,22 @@ namespace mmc
                 const u32 first = __shfl_sync(am, page, j);
                 const u32 tag = __shfl_sync(am, bytes, j);
                 const u32 end = umin(first + divup(tag, c.pagesize), c.numpages);
-                char* tail = c.pages + static_cast<u64>(first + 1u) * c.pagesize - 4u * masks;
-                for(u32 p = first; p < end; ++p, tail += c.pagesize)
-                    for(u32 w = rank; w < masks; w += g)
-                        st_rlx(reinterpret_cast<u32*>(tail) + w, 0u);
+                {
+                    const u32 P = c.pagesize;
+                    char* tail = c.pages + static_cast<u64>(first + 1u) * P - 4u * masks;
+                    for(u32 p = first; p < end; ++p, tail += P)
+                        for(u32 w = rank; w < masks; w += g)
+                            st_rlx(reinterpret_cast<u32*>(tail) + w, 0u);
+                }
                 for(u32 w = (first >> 5) + rank; 32u * w < end; w += g)
                     atomicOr(&walkmap(c.freemap, c.numpages)[w], word_span(w, first, end));
                 __threadfence();
                 __syncwarp(am);
                 u32 old = tag;
-#pragma unroll 4
+                u32* const chunksize = c.chunksize;
+#pragma unroll 1
                 for(u32 p = first + rank; p < end; p += g)
-                    old &= atomicCAS(&c.chunksize[p], tag, 0u);
+                    old &= atomicCAS(&chunksize[p], tag, 0u);
                 /* (old is what every lane's CASes returned: the ballot waits for them) */
                 if(__ballot_sync(am, old == tag) != 0u || old == 0u)
                     __syncwarp(am);
@@ -1970,14 +2068,19 @@ namespace mmc
                             MMC_STAT(h, MMC_STAT_PAGE_BASED);
                         const PageScan c{h.chunksize, h.freemap, h.state, h.pages, h.numpages, h.pagesize,
                                          h.reference_quirks};
+                        u32 run = large ? kPageSearch : kPageNone;
                         /* a whole warp's are served together */
                         if(active == 0xFFFFFFFFu)
                         {
-                            void* run = alloc_page_based_warp(c, large ? bytes : 0u);
-                            res = large ? run : res;
+                            PageCall call;
+                            call.c = c;
+                            call.bytes = large ? bytes : 0u;
+                            run = alloc_page_based_warp(&call);
                         }
-                        else if(large)
+                        if(run == kPageSearch)
                             res = alloc_page_based_concurrent(c, bytes);
+                        else if(run != kPageNone)
+                            res = page_data(h, run);
                     }
                 }
                 else if(large)
@@ -2073,9 +2176,8 @@ namespace mmc
                 if(runs)
                 {
                     const u32 which = __ballot_sync(active, owned && !chunk);
-                    dealloc_page_based_warp(PageScan{h.chunksize, h.freemap, h.state, h.pages, h.numpages, h.pagesize,
-                                                     h.reference_quirks},
-                                            h.maxOnPageMasks, active, which, page, chunksize);
+                    const PageScan c{h.chunksize, h.freemap, h.state, h.pages, h.numpages, h.pagesize, h.reference_quirks};
+                    dealloc_page_based_warp(&c, h.maxOnPageMasks, active, which, page, chunksize);
                 }
             }
             else if(owned && !chunk)
@@ -2106,17 +2208,18 @@ namespace mmc
             const u32 bytes = apply_padding(Ids::alignment(h), static_cast<u32>(bytes_in));
             /* one call of create for every form, so its code is in the kernel once */
             u32 req = bytes;
-            u32 active = 1u, threadcount = 0u, before = 0u, leader = 0u;
-            bool coalescible = false;
+            u32 active = 1u;
+            u32 joined = 0u; /* the lanes whose requests are one, 0: none are */
+            u32 before = 0u;
             if constexpr(Ids::warpSize > 1u)
                 active = calling_lanes();
             const u32 lane = Ids::laneid();
             if(Ids::coalesce && Ids::distribution(h) == MMC_DIST_XMALLOCSIMD)
             {
-                coalescible = bytes > 0u && bytes < (h.pagesize / 32u);
-                const u32 cmask = __ballot_sync(active, coalescible);
-                threadcount = static_cast<u32>(__popc(cmask));
-                if(threadcount > 1u)
+                const bool coalescible = bytes > 0u && bytes < (h.pagesize / 32u);
+                joined = __ballot_sync(active, coalescible);
+                joined = (joined & (joined - 1u)) != 0u ? joined : 0u;
+                if(joined != 0u)
                 {
                     /* exclusive prefix of the coalescible lanes' sizes, in lane order */
                     const u32 mine = coalescible ? bytes : 0u;
@@ -2135,7 +2238,7 @@ namespace mmc
                     else
                     {
 #pragma unroll 1
-                        for(u32 m = cmask; m != 0u; m &= m - 1u)
+                        for(u32 m = joined; m != 0u; m &= m - 1u)
                         {
                             const u32 src = static_cast<u32>(__ffs(static_cast<int>(m))) - 1u;
                             const u32 v = __shfl_sync(active, mine, static_cast<int>(src));
@@ -2144,20 +2247,18 @@ namespace mmc
                         }
                     }
                     const u32 total = __reduce_add_sync(active, mine);
-                    leader = static_cast<u32>(__ffs(static_cast<int>(cmask))) - 1u;
                     if(coalescible)
-                        req = (lane == leader) ? 16u + total : 0u;
+                        req = (joined & lanemask_lt()) == 0u ? 16u + total : 0u; /* the lowest asks for all */
                 }
-                else
-                    coalescible = false;
             }
             void* mem = create<Ids>(h, active, req);
             mem = handle_oom<Ids>(h, mem, req);
             if constexpr(Ids::warpSize > 1u)
             {
-                if(coalescible && lane == leader && mem != nullptr)
+                const bool part = ((joined >> lane) & 1u) != 0u;
+                if(part && (joined & lanemask_lt()) == 0u && mem != nullptr)
                 {
-                    st_rlx(static_cast<u32*>(mem), threadcount);
+                    st_rlx(static_cast<u32*>(mem), static_cast<u32>(__popc(joined)));
                     /* The count's sector is usually cold, and the store leaves it
                      * partly valid in L2: the frees' atomics on it would wait for
                      * the DRAM fill. Fetch it now, while the lanes use their parts. */
@@ -2173,11 +2274,11 @@ namespace mmc
                  * workload.) It also brings the lanes together again after their
                  * searches. */
                 __syncwarp(active);
-                if(threadcount > 1u)
+                if(joined != 0u)
                 {
-                    const unsigned long long base
-                        = __shfl_sync(active, reinterpret_cast<unsigned long long>(mem), static_cast<int>(leader));
-                    if(coalescible)
+                    const unsigned long long base = __shfl_sync(active, reinterpret_cast<unsigned long long>(mem),
+                                                                __ffs(static_cast<int>(joined)) - 1);
+                    if(part)
                         mem = base != 0ull ? reinterpret_cast<char*>(base) + 16u + before : nullptr;
                 }
             }

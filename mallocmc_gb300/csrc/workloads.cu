@@ -25,20 +25,6 @@ namespace
         z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
         return z ^ (z >> 31);
     }
-
-    /* The lanes of this warp that have a thread, of those whose index is below
-     * n (the caller's is) in a one-dimensional launch: known by arithmetic, for
-     * warp-wide operations at the top of a kernel. */
-    __device__ __forceinline__ uint32_t warp_lanes()
-    {
-        const uint32_t here = blockDim.x - (threadIdx.x & ~31u);
-        return here >= 32u ? 0xFFFFFFFFu : (1u << here) - 1u;
-    }
-    __device__ __forceinline__ uint32_t warp_lanes(uint32_t n)
-    {
-        const uint32_t below = n - (blockIdx.x * blockDim.x + (threadIdx.x & ~31u));
-        return warp_lanes() & (below >= 32u ? 0xFFFFFFFFu : (1u << below) - 1u);
-    }
 } // namespace
 
 /* One thread, SerialIds: the reference's CPU-serial semantics. */
@@ -231,53 +217,22 @@ __device__ __forceinline__ void stress_rounds(const mmc_device_handle& h, const 
     }
 }
 
-/* The rounds of a warp that asks for more than a page now and then: out of
- * line, the kernel's common rounds keep their registers. */
-template<uint32_t PATTERN, class Ids>
-__device__ __noinline__ StressCounts stress_rounds_large(const mmc_device_handle h, const mmc_stress_params p,
-                                                         const uint16_t* sizes, PatternPieces* pieces)
-{
-    StressCounts n{};
-    stress_rounds<PATTERN, Ids>(h, p, sizes, pieces, n);
-    return n;
-}
-
-/* malloc of a warp with a multi-page request among its lanes', out of line for the same reason */
-template<class Ids>
-__device__ __noinline__ void* malloc_large(const mmc_device_handle h, uint32_t bytes)
-{
-    return dv::malloc<Ids>(h, bytes);
-}
-
 /* Uniform stress: sizes[r * nthreads + t] or drawn from the seed. Launch
  * bounds of four 256-thread CTAs per SM (64 registers): that build measured
  * about 6 % faster on GB300 than the one without the bound.
- *
- * A warp whose requests all fit a page, the usual one, runs its rounds without
- * the multi-page path: with the call of it in the loop ptxas spilled 268 bytes
- * at that bound (6.95 against 5.80 ms on the uniform stress), and with both
- * loops inlined 348 (6.50 ms). It looks the size table through first, when
- * there is one, 200 bytes a thread of the benchmark's. */
+ * Ids without the multi-page path where the host knows that all sizes fit a
+ * page: 2.26 against 2.51 ms on per-thread patterns under the page reset, no
+ * difference on the uniform stress. Sizes from a table are not known to it. (Both
+ * forms in one kernel, the warp's choice, paid while the multi-page service took
+ * more registers than the bound. Now they take 6.8 ms on the uniform stress, the
+ * general one alone 6.2.) */
 template<uint32_t PATTERN, class Ids>
 __global__ void __launch_bounds__(256, 4) mmc_stress_kernel(mmc_device_handle h, mmc_stress_params p,
                                                          const uint16_t* sizes, unsigned long long* stats)
 {
     __shared__ PatternPieces pieces[PATTERN == MMC_PATTERN_WARP ? 8 : 1]; /* a warp's each */
-    uint32_t most = p.hi;
-    if(sizes != nullptr)
-    {
-        const uint32_t nthreads = gridDim.x * blockDim.x;
-        const uint16_t* mine = sizes + blockIdx.x * blockDim.x + threadIdx.x;
-        most = 0u;
-#pragma unroll 8
-        for(uint32_t r = 0; r < p.rounds; ++r)
-            most = max(most, static_cast<uint32_t>(mine[static_cast<uint64_t>(r) * nthreads]));
-    }
     StressCounts n{};
-    if(__any_sync(warp_lanes(), dv::apply_padding(Ids::alignment(h), most) > h.pagesize))
-        n = stress_rounds_large<PATTERN, Ids>(h, p, sizes, pieces);
-    else
-        stress_rounds<PATTERN, dv::SmallRequests<Ids>>(h, p, sizes, pieces, n);
+    stress_rounds<PATTERN, Ids>(h, p, sizes, pieces, n);
     if constexpr(PATTERN == MMC_PATTERN_WARP)
         n.csum += __shfl_xor_sync(0xFFFFFFFFu, n.other, 16);
     /* warp-aggregate the counters */
@@ -484,11 +439,7 @@ __global__ void __launch_bounds__(1024) mmc_verify_kernel(mmc_device_handle h, u
     uint32_t* p = nullptr;
     if(ALLOC)
     {
-        /* warps whose requests all fit a page keep clear of the multi-page path (see the stress kernel) */
-        if(__any_sync(warp_lanes(nthreads), dv::apply_padding(Ids::alignment(h), sizes[t]) > h.pagesize))
-            p = static_cast<uint32_t*>(malloc_large<Ids>(h, sizes[t]));
-        else
-            p = static_cast<uint32_t*>(dv::malloc<dv::SmallRequests<Ids>>(h, sizes[t]));
+        p = static_cast<uint32_t*>(dv::malloc<Ids>(h, sizes[t]));
         offsets[t] = p ? static_cast<int64_t>(reinterpret_cast<char*>(p) - h.pages) : -1;
         if(p)
             fill_words(p, sizes[t] / 4u, pattern);
@@ -527,6 +478,17 @@ __global__ void mmc_atomic_peak_kernel(uint32_t* buf, uint64_t mask, uint32_t it
     }
     if(returning && acc == 0x9E3779B9u)
         atomicAdd(sink, 1ull);
+}
+
+/* One instantiation per pattern mode: only the mode's code is in the kernel. */
+template<class Ids>
+static void launch_stress(const mmc_device_handle& h, const mmc_stress_params& p, const uint16_t* sizes,
+                          unsigned long long* stats, cudaStream_t s)
+{
+    if(p.write_pattern == MMC_PATTERN_WARP)
+        mmc_stress_kernel<MMC_PATTERN_WARP, Ids><<<p.blocks, p.threads_per_block, 0, s>>>(h, p, sizes, stats);
+    else
+        mmc_stress_kernel<MMC_PATTERN_THREAD, Ids><<<p.blocks, p.threads_per_block, 0, s>>>(h, p, sizes, stats);
 }
 
 extern "C" {
@@ -599,11 +561,10 @@ mmc_status mmc_run_stress(mmc_heap* heap, const mmc_stress_params* p, const uint
         return fail(MMC_ERR_ARG, "stress grid above 2^32 threads or more than 2^26 rounds");
     mmc_device_handle h;
     mmc_heap_device_handle(heap, &h);
-    /* One instantiation per pattern mode: only the mode's code is in the kernel. */
-    MMC_DISPATCH_IDS(h, if(p->write_pattern == MMC_PATTERN_WARP) mmc_stress_kernel<MMC_PATTERN_WARP, Ids>
-                            <<<p->blocks, p->threads_per_block, 0, as_stream(stream)>>>(h, *p, sizes, stats);
-                     else mmc_stress_kernel<MMC_PATTERN_THREAD, Ids>
-                         <<<p->blocks, p->threads_per_block, 0, as_stream(stream)>>>(h, *p, sizes, stats));
+    if(sizes == nullptr && dv::apply_padding(h.dataAlignment, p->hi) <= h.pagesize)
+        MMC_DISPATCH_IDS(h, launch_stress<dv::SmallRequests<Ids>>(h, *p, sizes, stats, as_stream(stream)));
+    else
+        MMC_DISPATCH_IDS(h, launch_stress<Ids>(h, *p, sizes, stats, as_stream(stream)));
     return cuda_check(cudaGetLastError(), "stress kernel");
 }
 
