@@ -668,8 +668,6 @@ namespace mmc
                     /* the region has no page left to try: on to the next one to walk */
                     if(walking && (Ids::warpSize == 1u || !batched || !room))
                     {
-                        if(level == 255u)
-                            level = ld_rlx(&h.regions[region]);
                         if(level + 1u <= R && (Ids::warpSize == 1u || checklevel <= R))
                             atomicCAS(&h.regions[region], level, level + 1u);
                         MMC_STAT(h, MMC_STAT_REGION_FAIL);
@@ -734,6 +732,9 @@ namespace mmc
                     /* the counter as it was looked at, up to eight regions ago: of
                      * several walks that fail here together one raises it */
                     level = static_cast<u32>(ahead) & 255u;
+                    /* of large regions a byte does not hold the counter that decides */
+                    if(go && level == 255u && checklevel > 255u)
+                        level = ld_rlx(&h.regions[region]);
                     walking = go && level < checklevel;
                     masks = batched;
                     todo = 0u;
