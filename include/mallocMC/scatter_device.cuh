@@ -2022,9 +2022,10 @@ namespace mmc
          * the work: a run's page tails, chunk sizes and bitmap words spread
          * over them. One lane alone zeroed 32 words per page and issued a
          * CAS per page: half of a wave's 920 blocks freed on a 512 MiB heap
-         * took 202 us. The CASes have returned before the bits are set: a bit
-         * set ahead of its CAS could be taken by the server, whose claim then
-         * fails and leaves the page's bit clear for good. */
+         * took 202 us. Every lane's CASes are performed before any lane sets a
+         * bit, by the fence and the barrier that all lanes pass: a bit set ahead
+         * of its CAS could be taken by the server, whose claim then fails and
+         * leaves the page's bit clear for good. */
         __device__ __noinline__ inline void dealloc_page_based_warp(const volatile PageScan* context, u32 masks, u32 am,
                                                                     u32 runs, u32 page, u32 bytes)
         {
@@ -2048,14 +2049,12 @@ namespace mmc
                     atomicOr(&walkmap(c.freemap, c.numpages)[w], word_span(w, first, end));
                 __threadfence();
                 __syncwarp(am);
-                u32 old = tag;
                 u32* const chunksize = c.chunksize;
 #pragma unroll 1
                 for(u32 p = first + rank; p < end; p += g)
-                    old &= atomicCAS(&chunksize[p], tag, 0u);
-                /* (old is what every lane's CASes returned: the ballot waits for them) */
-                if(__ballot_sync(am, old == tag) != 0u || old == 0u)
-                    __syncwarp(am);
+                    atomicCAS(&chunksize[p], tag, 0u);
+                __threadfence();
+                __syncwarp(am);
                 for(u32 w = (first >> 5) + rank; 32u * w < end; w += g)
                     atomicOr(&c.freemap[w], word_span(w, first, end));
                 if(rank == 0u)
