@@ -17,7 +17,8 @@
  *     lanes that are active at the call, not shared-memory counters;
  *   - every spin is bounded: the page-based mutex gives up after a fixed
  *     number of backed-off tries, records MMC_DEVERR_TIMEOUT and returns NULL;
- *     the bit-claim retry loop gives up after MMC_USESPOT_MAX_TRIES.
+ *     a wait for the multi-page service ends in the lock-free search; the
+ *     bit-claim retry loop gives up after MMC_USESPOT_MAX_TRIES.
  * Thread-id sources are a template parameter: GpuIds reads %laneid/%warpid/
  * %smid (mallocMC_utils.hpp:91-150); SerialIds is the reference CPU backend
  * (all zero, warp size 1), which makes one device thread reproduce the
@@ -34,6 +35,11 @@
 #endif
 #ifndef MMC_MUTEX_MAX_SPINS
 #define MMC_MUTEX_MAX_SPINS (1u << 22)
+#endif
+/* looks at the multi-page service without a ticket served, one to two
+ * microseconds each (a batch reads the heap's free-page bitmap twice at most) */
+#ifndef MMC_SERVICE_MAX_IDLE
+#define MMC_SERVICE_MAX_IDLE (1u << 20)
 #endif
 
 /* Mutable heap words, each on its own 128-byte line. */
@@ -58,12 +64,13 @@ struct mmc_heap_state
 struct mmc_page_service
 {
     uint32_t lock; /* held by the warp that serves */
-    uint32_t pad0[31];
+    uint32_t closed; /* set when a wait ran out: requests take the lock-free search */
+    uint32_t pad0[30];
     uint32_t tail; /* tickets handed out */
     uint32_t pad1[31];
     uint32_t head; /* tickets served; the lock's holder moves it */
     uint32_t pad2[31];
-    uint32_t ring[MMC_PAGE_RING]; /* 0: idle; kPageAsk | pages: waiting; else the answer */
+    uint32_t ring[MMC_PAGE_RING]; /* 0: idle; kPageAsk or kPageGone | pages; kPageAnswer | page */
 };
 
 #ifdef MMC_DEVICE_STATS
@@ -1416,14 +1423,14 @@ namespace mmc
          * Partial warps and requests above kServiceMaxPages keep the
          * lock-free search. */
         constexpr u32 kPageAsk = 0x80000000u; /* ring word of a waiting request */
-        constexpr u32 kPageGone = 0xC0000000u; /* ring word of a request given up */
+        constexpr u32 kPageGone = 0xC0000000u; /* ring word of a request given up: | pages */
         constexpr u32 kPageAnswer = 0x40000000u; /* ring word of an answer: | first page */
         constexpr u32 kPageNone = 0x3FFFFFFFu; /* answer's page when there is no run */
         constexpr u32 kPageSearch = 0x7FFFFFFFu; /* "use the lock-free search", not in the ring */
         constexpr u32 kServiceMaxPages = 1024u; /* 32 claims per lane, remembered in one word */
         constexpr u32 kServiceRetries = 4u; /* runs lost to chunk pages before the lock-free search is used */
 
-        __device__ __forceinline__ mmc_page_service* page_service(mmc_heap_state* state)
+        __host__ __device__ __forceinline__ mmc_page_service* page_service(mmc_heap_state* state)
         {
             return reinterpret_cast<mmc_page_service*>(state + 1);
         }
@@ -1492,6 +1499,8 @@ namespace mmc
             u32 stage;
             u32 ticket;
             u32 polls;
+            u32 seen; /* the tickets served, as lane 0 last saw them, */
+            u32 idle; /* and how many looks ago that changed */
             u32 run; /* first page of the run found, kPageNone: none */
             /* the batch it serves */
             u32 head;
@@ -1736,34 +1745,29 @@ namespace mmc
             mmc_page_service* sv = page_service(req.c.state);
             const u32 lane = GpuIds::laneid();
             const u32 head = req.head;
+            /* the words, read together with the tail: one a ticket has by then
+             * and that holds no request yet is read again */
+            u32 v[kServiceSlots];
+#pragma unroll
+            for(u32 s = 0; s < kServiceSlots; ++s)
+                v[s] = ld_rlx(&sv->ring[(head + 32u * s + lane) & (MMC_PAGE_RING - 1u)]);
             const u32 have = __shfl_sync(kFull, umin(ld_rlx(&sv->tail) - head, kServiceBatch), 0);
             u32 taken = have;
-#pragma unroll 1
-            for(u32 k = 0; k < kServiceWords; k += 2u)
+#pragma unroll
+            for(u32 s = 0; s < kServiceSlots; ++s)
             {
-                u32 v[4];
-#pragma unroll
-                for(u32 j = 0; j < 4u; ++j)
-                {
-                    const u32 i = 64u * k + 32u * j + lane;
-                    v[j] = i < have ? ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]) : 0u;
-                }
-#pragma unroll
-                for(u32 j = 0; j < 4u; ++j)
-                {
-                    const u32 i = 64u * k + 32u * j + lane;
+                const u32 i = 32u * s + lane;
 #pragma unroll 1
-                    for(u32 spin = 0; i < taken && (v[j] & kPageAsk) == 0u; ++spin)
-                    {
-                        v[j] = ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]);
-                        if(spin == 64u)
-                            taken = i;
-                    }
-                    /* given up: kept as 0xFFFF until it is known whether the batch has it */
-                    v[j] = v[j] == kPageGone ? 0xFFFFu : v[j] & 0xFFFFu;
+                for(u32 spin = 0; i < taken && (v[s] & kPageAsk) == 0u; ++spin)
+                {
+                    v[s] = ld_rlx(&sv->ring[(head + i) & (MMC_PAGE_RING - 1u)]);
+                    if(spin == 64u)
+                        taken = i;
                 }
-                req.w[k] = v[0] | v[1] << 16;
-                req.w[k + 1u] = v[2] | v[3] << 16;
+                /* given up: kept as 0xFFFF until it is known whether the batch has it */
+                v[s] = v[s] >= kPageGone ? 0xFFFFu : v[s] & 0xFFFFu;
+                if((s & 1u) != 0u)
+                    req.w[s / 2u] = v[s - 1u] | v[s] << 16;
             }
             taken = __reduce_min_sync(kFull, taken);
             u32 asked = 0u, sum = 0u;
@@ -1796,14 +1800,40 @@ namespace mmc
             /* every lane's bit clears are performed before any answer is seen */
             __threadfence();
             __syncwarp();
-#pragma unroll 1
-            for(u32 m = req.asked; m != 0u; m &= m - 1u)
+            u32 was[kServiceSlots];
+            const u32 asked = req.asked;
+#pragma unroll
+            for(u32 s = 0; s < kServiceSlots; ++s)
             {
-                const u32 s = static_cast<u32>(__ffs(static_cast<int>(m))) - 1u;
                 const bool none = ((req.w[s / 2u] >> (16u * (s & 1u))) & 0xFFFFu) != 0u;
-                const u32 page = req.page[s];
-                st_rlx(&sv->ring[(head + 32u * s + lane) & (MMC_PAGE_RING - 1u)], kPageAnswer | (none ? +kPageNone : page));
+                const u32 answer = kPageAnswer | (none ? +kPageNone : +req.page[s]);
+                was[s] = ((asked >> s) & 1u) != 0u
+                    ? atomicExch(&sv->ring[(head + 32u * s + lane) & (MMC_PAGE_RING - 1u)], answer)
+                    : 0u;
             }
+            u32 gone = 0u; /* those whose askers have left since the batch was taken */
+#pragma unroll
+            for(u32 s = 0; s < kServiceSlots; ++s)
+                if(was[s] >= kPageGone)
+                {
+                    /* (its half now says what goes back: the pages of a run that was placed) */
+                    const u32 v = req.w[s / 2u], shift = 16u * (s & 1u);
+                    req.w[s / 2u] = (v >> shift & 0xFFFFu) != 0u ? v & ~(0xFFFFu << shift) : v | (was[s] & 0xFFFFu) << shift;
+                    gone |= 1u << s;
+                }
+#pragma unroll 1
+            for(; gone != 0u; gone &= gone - 1u)
+            {
+                const u32 s = static_cast<u32>(__ffs(static_cast<int>(gone))) - 1u;
+                const u32 n = (req.w[s / 2u] >> (16u * (s & 1u))) & 0xFFFFu;
+                if(n != 0u)
+                {
+                    freemap_range(req.c.freemap, req.page[s], n, true);
+                    atomicMax(&req.c.state->firstFreePageBased, req.page[s] + n - 1u);
+                }
+                st_rlx(&sv->ring[(head + 32u * s + lane) & (MMC_PAGE_RING - 1u)], 0u); /* idle again */
+            }
+            __syncwarp();
             req.head = head + req.taken;
             if(lane == 0u)
                 st_rlx(&sv->head, head + req.taken);
@@ -1815,27 +1845,38 @@ namespace mmc
             const u32 asking = __ballot_sync(0xFFFFFFFFu, call->stage == kAsks);
             if(asking == 0u)
                 return false;
+            mmc_page_service* sv = page_service(call->c.state);
             u32 ticket = 0u;
+            const u32 closed = __shfl_sync(0xFFFFFFFFu, ld_rlx(&sv->closed), 0);
+            if(closed != 0u)
+                return false;
             if(GpuIds::laneid() == 0u)
-                ticket = atomicAdd(&page_service(call->c.state)->tail, static_cast<u32>(__popc(asking)));
+                ticket = atomicAdd(&sv->tail, static_cast<u32>(__popc(asking)));
             ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0) + static_cast<u32>(__popc(asking & lanemask_lt()));
             if(call->stage == kAsks)
                 call->stage = kTicket; /* (its run is kPageNone; the others' may have runs already) */
             call->ticket = ticket;
-            call->polls = 0u;
+            call->polls = call->idle = call->seen = 0u;
             return true;
         }
 
-        /* One look at the ring by a waiting warp: 0 when all its requests are
-         * answered, 1 to look again, 2 when it has taken the lock to serve. */
+        /* One look at the ring by a waiting warp: 0 when it waits no more, 1 to
+         * look again, 2 when it has taken the lock to serve.
+         *
+         * A wait ends when no ticket has been served for MMC_SERVICE_MAX_IDLE
+         * looks. (Not after a time of its own: a full grid's requests on a heap
+         * that runs out wait for a thousand batches.) The warp that sees it
+         * closes the service until the heap is initialised again; it and all
+         * that wait give their requests up and search lock-free, as every later
+         * request does. A ticket given up unwritten stays a hole in the ring,
+         * which no server passes: hence the closing. A written word is given up
+         * by a CAS, which fails when its answer is there. */
         __device__ __noinline__ inline u32 page_service_poll(volatile PageCall* call)
         {
             constexpr u32 kFull = 0xFFFFFFFFu;
             mmc_page_service* sv = page_service(call->c.state);
             const u32 ticket = call->ticket;
             u32* word = &sv->ring[ticket & (MMC_PAGE_RING - 1u)];
-            const u32 polls = call->polls;
-            const bool late = polls > MMC_MUTEX_MAX_SPINS;
             u32 stage = call->stage;
             if(stage == kTicket)
             {
@@ -1846,8 +1887,6 @@ namespace mmc
                     st_rlx(word, kPageAsk | divup(call->bytes, call->c.pagesize));
                     stage = kWaits;
                 }
-                else if(late)
-                    stage = kAnswered;
             }
             else if(stage == kWaits)
             {
@@ -1858,31 +1897,58 @@ namespace mmc
                     st_rlx(word, 0u);
                     stage = kAnswered;
                 }
-                else if(late && atomicCAS(word, v, kPageGone) == v)
-                    stage = kAnswered;
             }
-            if(late)
-                atomicOr(&call->c.state->error_flags, MMC_DEVERR_TIMEOUT);
+            u32 look = 0u; /* 1: again, 2: the lock is this warp's, 3: the service is closed */
+            if(__any_sync(kFull, stage == kTicket || stage == kWaits))
+            {
+                look = 1u;
+                if(GpuIds::laneid() == 0u)
+                {
+                    const u32 lock = ld_rlx(&sv->lock), head = ld_rlx(&sv->head), closed = ld_rlx(&sv->closed);
+                    const u32 idle = head == call->seen ? call->idle + 1u : 0u;
+                    call->seen = head;
+                    call->idle = idle;
+                    if(closed != 0u || idle > MMC_SERVICE_MAX_IDLE)
+                    {
+                        look = 3u;
+                        if(atomicExch(&sv->closed, 1u) == 0u)
+                            atomicOr(&call->c.state->error_flags, MMC_DEVERR_TIMEOUT);
+                    }
+                    else if(lock == 0u)
+                        look = atomicCAS(&sv->lock, 0u, 1u) == 0u ? 2u : 1u;
+                }
+                look = __shfl_sync(kFull, look, 0);
+                if(look == 3u)
+                {
+                    if(stage == kWaits)
+                    {
+                        const u32 asked = kPageAsk | divup(call->bytes, call->c.pagesize);
+                        const u32 v = atomicCAS(word, asked, asked | kPageGone);
+                        if(v != asked)
+                        {
+                            call->run = v & kPageNone;
+                            st_rlx(word, 0u);
+                            stage = kAnswered;
+                        }
+                    }
+                    if(stage == kTicket || stage == kWaits)
+                        stage = kSearches;
+                    look = 0u;
+                }
+            }
             call->stage = stage;
-            call->polls = polls + 1u;
-            if(!__any_sync(kFull, stage == kTicket || stage == kWaits))
+            if(look == 1u)
             {
-                /* what the server did to the bitmap is performed before what follows */
-                __threadfence();
-                return 0u;
+                const u32 polls = call->polls;
+                call->polls = polls + 1u;
+                if(polls > 1u)
+                    __nanosleep(umin(64u << umin(polls, 5u), 1024u));
             }
-            u32 lock = 1u;
-            if(GpuIds::laneid() == 0u && ld_rlx(&sv->lock) == 0u)
-                lock = atomicCAS(&sv->lock, 0u, 1u);
-            if(__shfl_sync(kFull, lock, 0) == 0u)
-            {
+            else /* the lock is taken, or answers are read: what servers did is performed before what follows */
                 __threadfence();
+            if(look == 2u)
                 call->head = ld_rlx(&sv->head);
-                return 2u;
-            }
-            if(polls > 1u)
-                __nanosleep(umin(64u << umin(polls, 5u), 1024u));
-            return 1u;
+            return look;
         }
 
         /* Serve what waits, batch by batch; the warp (whole) holds the lock. */
@@ -1907,7 +1973,6 @@ namespace mmc
                 }
                 page_service_answer(call);
             }
-
             __threadfence();
             __syncwarp();
             if(GpuIds::laneid() == 0u)

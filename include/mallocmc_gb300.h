@@ -46,7 +46,9 @@ typedef enum mmc_status
 #define MMC_OOM_FLAG 1       /* BadAllocException's device branch without the trap: sets MMC_DEVERR_OOM, returns NULL */
 
 /* Device error bits reported by mmc_heap_error. */
-#define MMC_DEVERR_TIMEOUT 0x1u  /* the page-based mutex wait hit its iteration bound */
+#define MMC_DEVERR_TIMEOUT 0x1u  /* the page-based mutex wait hit its iteration bound, or a wait for the
+                                    multi-page service did, which is closed since (requests are served
+                                    without it) */
 #define MMC_DEVERR_BADFREE 0x2u  /* free of a pointer outside the heap or on an unformatted page */
 #define MMC_DEVERR_OOM 0x4u      /* an allocation failed under MMC_OOM_FLAG */
 #define MMC_DEVERR_BADCMD 0x8u   /* a serving tick skipped a command (slot beyond the table, unknown kind,

@@ -270,6 +270,31 @@ namespace
         }
     }
 
+    /* Every thread asks for three pages, whole warps together, and marks the
+     * first and last word; counts: blocks got, NULLs. */
+    __global__ void threePagesKernel(ScatterAllocator::AllocatorHandle h, unsigned** blocks, unsigned* counts)
+    {
+        const Acc acc{};
+        const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
+        unsigned* p = static_cast<unsigned*>(h.malloc(acc, 3 * 4096));
+        blocks[id] = p;
+        atomicAdd(&counts[p != nullptr ? 0 : 1], 1u);
+        if(p != nullptr)
+            p[0] = p[3 * 1024 - 1] = id;
+    }
+
+    __global__ void freeThreePagesKernel(ScatterAllocator::AllocatorHandle h, unsigned** blocks, unsigned* wrong)
+    {
+        const Acc acc{};
+        const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
+        unsigned* p = blocks[id];
+        if(p == nullptr)
+            return;
+        if(p[0] != id || p[3 * 1024 - 1] != id)
+            atomicAdd(wrong, 1u);
+        h.free(acc, p);
+    }
+
     int report(const std::exception& e)
     {
         std::fprintf(stderr, "mmcx: %s\n", e.what());
@@ -425,6 +450,56 @@ int mmcx_churn(int device, unsigned blocks, unsigned threads, unsigned rounds, u
         *flags = alloc.errorFlags();
         cudaFree(d_counts);
         return refused ? 3 : (cudaDeviceSynchronize() == cudaSuccess ? 0 : 2);
+    }
+    catch(const std::exception& e)
+    {
+        return report(e);
+    }
+}
+
+/* Multi-page requests of 256 threads, twice, on a heap whose service is left by
+ * the host as a warp that gave up might leave it: 0: locked by nobody who
+ * serves; 1: a ticket drawn and never written; 2: a request given up, which a
+ * server passes; 3: untouched. out[6] = {blocks got, NULLs (both times), words
+ * wrong, whether the service is closed, pages still claimed, device error bits}. */
+int mmcx_service_wait(int device, int state, unsigned* out)
+{
+    try
+    {
+        cudaSetDevice(device);
+        ScatterAllocator alloc(device, nullptr, 1U * 1024U * 1024U * 1024U);
+        const auto handle = alloc.getAllocatorHandle();
+        const mmc_device_handle& d = handle.devAllocator;
+        mmc_page_service* service = mmc::dev::page_service(d.state);
+        const unsigned one = 1u, gone = mmc::dev::kPageGone | 3u;
+        if(state == 0)
+            cudaMemcpy(&service->lock, &one, sizeof(one), cudaMemcpyHostToDevice);
+        if(state == 1 || state == 2)
+            cudaMemcpy(&service->tail, &one, sizeof(one), cudaMemcpyHostToDevice);
+        if(state == 2)
+            cudaMemcpy(&service->ring[0], &gone, sizeof(gone), cudaMemcpyHostToDevice);
+        const unsigned threads = 64, grid = 4;
+        unsigned** d_blocks = nullptr;
+        unsigned* d_counts = nullptr;
+        cudaMalloc(&d_blocks, sizeof(unsigned*) * threads * grid);
+        cudaMalloc(&d_counts, 3 * sizeof(unsigned));
+        cudaMemset(d_counts, 0, 3 * sizeof(unsigned));
+        for(int again = 0; again < 2; ++again)
+        {
+            threePagesKernel<<<grid, threads>>>(handle, d_blocks, d_counts);
+            freeThreePagesKernel<<<grid, threads>>>(handle, d_blocks, d_counts + 2);
+        }
+        cudaMemcpy(out, d_counts, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost);
+        cudaMemcpy(out + 3, &service->closed, sizeof(unsigned), cudaMemcpyDeviceToHost);
+        std::vector<uint32_t> chunksizes(d.numpages);
+        cudaMemcpy(chunksizes.data(), d.chunksize, sizeof(uint32_t) * d.numpages, cudaMemcpyDeviceToHost);
+        out[4] = 0u;
+        for(const uint32_t c : chunksizes)
+            out[4] += c != 0u ? 1u : 0u;
+        out[5] = alloc.errorFlags();
+        cudaFree(d_blocks);
+        cudaFree(d_counts);
+        return cudaDeviceSynchronize() == cudaSuccess ? 0 : 2;
     }
     catch(const std::exception& e)
     {
