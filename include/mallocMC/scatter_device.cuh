@@ -609,10 +609,10 @@ namespace mmc
          * counters are looked at eight regions ahead, so a stretch of regions
          * skipped as 3/4 full costs one round trip and one step per eight;
          * read with them, a word of the map of pages outside multi-page runs
-         * has both passes skip the regions that runs fill as well. (The 32 GiB fragmentation run's two
-         * waves up to its first NULL: 800 and 50 to 1140 ms a region at a
-         * time, 850 and 915 by the counters alone, 226 and 550 so; the whole
-         * run 2.2 to 3.4 s, now 1.3 s.) Alone on the heap every page gets
+         * has both passes skip the regions that runs fill as well. (The 32 GiB
+         * fragmentation run's two waves up to its first NULL: 800 and 50 to
+         * 1140 ms a region at a time, 850 and 915 by the counters alone, 226 and
+         * 550 so; the whole run 2.2 to 3.4 s, now 1.3 s.) Alone on the heap every page gets
          * the reference's outcome, in the reference's order.
          *
          * The counters: the reference counts every failed walk, whatever size
@@ -634,10 +634,13 @@ namespace mmc
          * 100 to 180 KB of code, and instruction fetch was the first stall of
          * the stress and batched kernels.
          *
-         * The lanes of a warp do not wait for one another in here. Walking
-         * step by step together they took fewer instructions (4.99 against
-         * 5.8 ms on the uniform stress), but a few launches in a hundred of a
-         * 16 to 256 byte stress did not end. */
+         * The lanes of a warp do not wait for one another in here: no step
+         * names a mask, so a lane's walk ends by itself, after the pages of
+         * 2 * numregions regions. (A form whose lanes stepped together, by a
+         * vote over lanes read inside this branch, took 4.99 ms on the uniform
+         * stress where this one takes 6.2, but a few launches in a hundred of a
+         * 16 to 256 byte stress did not end. What masks read in branches did
+         * elsewhere is at calling_lanes; the form was not run again.) */
         template<class Ids>
         __device__ __forceinline__ void* alloc_chunked_walk(const mmc_device_handle& h, u32 bytes, u32 minAllocation,
                                                             u32 maxchunksize, u32 start, u32 level)
