@@ -2498,9 +2498,13 @@ namespace mmc
 
         /* handle.getAvailableSlots (device_allocator.hpp:98-106 ->
          * getAvailableSlotsAccelerator, Scatter.hpp:1311-1352): the lanes active
-         * at the call share the scan and all of them receive the count. Unlike
-         * the reference it needs no block-wide barrier, so any subset of threads
-         * may call it. slotSize is padded first (device_allocator.hpp:103). */
+         * at the call with one size share its scan and all of them receive the
+         * count. Unlike the reference it needs no block-wide barrier, so any
+         * subset of threads may call it; and lanes that come with different sizes
+         * (also of one source line: the lanes of a loop meet in different rounds of
+         * it) are parted first, where a scan over all of them would add up pages
+         * counted for one size and the other. slotSize is padded first
+         * (device_allocator.hpp:103). */
         template<class Ids>
         __device__ unsigned available_slots(const mmc_device_handle& h, size_t slotSize_in)
         {
@@ -2510,7 +2514,7 @@ namespace mmc
             u32 active = 1u, rank = 0u, nact = 1u;
             if(Ids::warpSize > 1u)
             {
-                active = calling_lanes();
+                active = __match_any_sync(calling_lanes(), slot);
                 nact = static_cast<u32>(__popc(active));
                 rank = static_cast<u32>(__popc(active & lanemask_lt()));
             }

@@ -270,6 +270,17 @@ namespace
         }
     }
 
+    /* Thread t asks for the free slots of sizes[t], `ahead` rounds of a loop
+     * behind or ahead of its neighbours'. */
+    __global__ void slotsOfSizesKernel(ScatterAllocator::AllocatorHandle h, const unsigned* sizes, unsigned ahead,
+                                       unsigned* slots)
+    {
+        const Acc acc{};
+        const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
+        for(unsigned r = 0; r <= (ahead != 0u ? id % ahead : 0u); ++r)
+            slots[id] = h.getAvailableSlots(acc, sizes[id]);
+    }
+
     /* Every thread asks for three pages, whole warps together, and marks the
      * first and last word; counts: blocks got, NULLs. */
     __global__ void threePagesKernel(ScatterAllocator::AllocatorHandle h, unsigned** blocks, unsigned* counts)
@@ -450,6 +461,38 @@ int mmcx_churn(int device, unsigned blocks, unsigned threads, unsigned rounds, u
         *flags = alloc.errorFlags();
         cudaFree(d_counts);
         return refused ? 3 : (cudaDeviceSynchronize() == cudaSuccess ? 0 : 2);
+    }
+    catch(const std::exception& e)
+    {
+        return report(e);
+    }
+}
+
+/* Device-side slot counts of n sizes (n a multiple of 32), a thread each, on a
+ * heap partly used, and the host's counts of the same sizes. */
+int mmcx_slots_of_sizes(int device, const unsigned* sizes, unsigned n, unsigned ahead, unsigned* slots, unsigned* host)
+{
+    try
+    {
+        cudaSetDevice(device);
+        ScatterAllocator alloc(device, nullptr, 300U * 1024U * 1024U);
+        unsigned** d_blocks = nullptr;
+        unsigned *d_counts = nullptr, *d_sizes = nullptr, *d_slots = nullptr;
+        cudaMalloc(&d_blocks, sizeof(unsigned*) * 96);
+        cudaMalloc(&d_counts, 2 * sizeof(unsigned));
+        cudaMalloc(&d_sizes, sizeof(unsigned) * n);
+        cudaMalloc(&d_slots, sizeof(unsigned) * n);
+        threePagesKernel<<<1, 96>>>(alloc.getAllocatorHandle(), d_blocks, d_counts);
+        cudaMemcpy(d_sizes, sizes, sizeof(unsigned) * n, cudaMemcpyHostToDevice);
+        slotsOfSizesKernel<<<n / 32u, 32>>>(alloc.getAllocatorHandle(), d_sizes, ahead, d_slots);
+        cudaMemcpy(slots, d_slots, sizeof(unsigned) * n, cudaMemcpyDeviceToHost);
+        for(unsigned i = 0; i < n; ++i)
+            host[i] = alloc.getAvailableSlots(device, nullptr, sizes[i]);
+        cudaFree(d_blocks);
+        cudaFree(d_counts);
+        cudaFree(d_sizes);
+        cudaFree(d_slots);
+        return cudaDeviceSynchronize() == cudaSuccess ? 0 : 2;
     }
     catch(const std::exception& e)
     {
