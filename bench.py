@@ -170,12 +170,12 @@ def batched_algorithmic_atomics(jobs, pagesize: int) -> dict:
 # a 2 GiB heap with 20 rounds (profiles/mmc_stress_kernel_uniform_2GiB_20rounds.md):
 # the partial lines at the blocks' ends (their whole lines are discarded from L2
 # before the free) and the metadata, so it scales with pairs.
-STRESS_DRAM_BYTES_PER_PAIR = 141.0
+STRESS_DRAM_BYTES_PER_PAIR = 158.0
 # L2 atomic requests per pair counted by ncu (lts__t_requests_srcunit_tex_op_atom*
 # + op_red) in the same capture: below the reference algorithm's 4.72 because a
 # formatted page's chunk size is loaded instead of CAS'd and same-size lanes
 # share one reservation.
-STRESS_NCU_ATOMICS_PER_PAIR = 3.91
+STRESS_NCU_ATOMICS_PER_PAIR = 3.92
 # L2 atomic requests per pair of the batched workload's persistent kernel, from
 # an ncu capture on the tuned geometry (profiles/mmc_batch_kernel_512jobs_4GiB.md).
 BATCH_NCU_ATOMICS_PER_PAIR = 0.206

@@ -640,7 +640,7 @@ namespace mmc
          * names a mask, so a lane's walk ends by itself, after the pages of
          * 2 * numregions regions. (A form whose lanes stepped together, by a
          * vote over lanes read inside this branch, took 4.99 ms on the uniform
-         * stress where this one takes 6.2, but a few launches in a hundred of a
+         * stress where this one takes 6.1, but a few launches in a hundred of a
          * 16 to 256 byte stress did not end. What masks read in branches did
          * elsewhere is at calling_lanes; the form was not run again.) */
         template<class Ids>

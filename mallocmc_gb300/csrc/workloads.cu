@@ -357,8 +357,7 @@ __device__ __forceinline__ unsigned long long frag_check_tags(const char* p, uin
     return bad;
 }
 
-/* Bounded to 64 registers, four blocks per SM: unbounded, the multi-page
- * service takes 103 and two blocks fit. */
+/* Bounded to 64 registers, four blocks per SM (it takes 63). */
 template<class Ids>
 __global__ void __launch_bounds__(256, 4) mmc_fill_kernel(mmc_device_handle h, mmc_frag_params p, uint64_t wave,
                                                        void** ptrs, uint32_t* sizes, uint64_t capacity,
@@ -426,8 +425,7 @@ __global__ void mmc_verify_list_kernel(void* const* ptrs, const uint32_t* sizes,
 }
 
 /* Verify workload: malloc(sizes[t]); write u32 (t ^ seed); optionally verify
- * and free. Bounded to 64 registers (blocks of up to 1024 threads): unbounded,
- * the multi-page service takes 105. */
+ * and free. Blocks of up to 1024 threads: 64 registers. */
 template<bool ALLOC, bool FREE, class Ids>
 __global__ void __launch_bounds__(1024) mmc_verify_kernel(mmc_device_handle h, uint32_t nthreads, const uint32_t* sizes, uint32_t seed,
                                   int64_t* offsets, unsigned long long* errors)
