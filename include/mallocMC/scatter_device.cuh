@@ -1952,7 +1952,7 @@ namespace mmc
             else /* the lock is taken, or answers are read: what servers did is performed before what follows */
                 __threadfence();
             if(look == 2u)
-                call->head = ld_rlx(&sv->head);
+                call->head = __shfl_sync(kFull, ld_rlx(&sv->head), 0);
             return look;
         }
 
@@ -1965,7 +1965,9 @@ namespace mmc
                 const u32 sum = page_service_take(call);
                 if(call->taken == 0u)
                     break;
-                call->entry = ld_rlx(&call->c.state->firstFreePageBased);
+                /* one lane's reading for all: frees raise the hint meanwhile, and lanes
+                 * with hints of their own clear bits of pages that no run has */
+                call->entry = __shfl_sync(0xFFFFFFFFu, ld_rlx(&call->c.state->firstFreePageBased), 0);
                 /* (from the reference's wrapped hint searches visit no page) */
                 if(sum != 0u && call->entry != 0xFFFFFFFFu && !page_service_stretch(call, sum))
                 {

@@ -306,6 +306,19 @@ namespace
         h.free(acc, p);
     }
 
+    /* Free pages that no multi-page search would find: their bits in the free-page
+     * map are clear. */
+    unsigned hidden_pages(const mmc_device_handle& d)
+    {
+        std::vector<uint32_t> sizes(d.numpages), map(d.numpages / 32u + 1u);
+        cudaMemcpy(sizes.data(), d.chunksize, sizeof(uint32_t) * sizes.size(), cudaMemcpyDeviceToHost);
+        cudaMemcpy(map.data(), d.freemap, sizeof(uint32_t) * map.size(), cudaMemcpyDeviceToHost);
+        unsigned hidden = 0;
+        for(uint32_t p = 0; p < d.numpages; ++p)
+            hidden += sizes[p] == 0u && ((map[p / 32u] >> (p % 32u)) & 1u) == 0u ? 1u : 0u;
+        return hidden;
+    }
+
     int report(const std::exception& e)
     {
         std::fprintf(stderr, "mmcx: %s\n", e.what());
@@ -461,6 +474,33 @@ int mmcx_churn(int device, unsigned blocks, unsigned threads, unsigned rounds, u
         *flags = alloc.errorFlags();
         cudaFree(d_counts);
         return refused ? 3 : (cudaDeviceSynchronize() == cudaSuccess ? 0 : 2);
+    }
+    catch(const std::exception& e)
+    {
+        return report(e);
+    }
+}
+
+/* The same, `times` launches on one heap; *hidden: free pages hidden at the end,
+ * all blocks freed. */
+int mmcx_churn_map(int device, unsigned times, unsigned blocks, unsigned threads, unsigned lo, unsigned hi,
+                   unsigned long long* counts, unsigned* hidden)
+{
+    try
+    {
+        cudaSetDevice(device);
+        ChurnAllocator alloc(device, nullptr, 1U * 1024U * 1024U * 1024U);
+        const auto pool = alloc.getHeapLocations().at(0);
+        unsigned long long* d_counts = nullptr;
+        cudaMalloc(&d_counts, 4 * sizeof(unsigned long long));
+        cudaMemset(d_counts, 0, 4 * sizeof(unsigned long long));
+        for(unsigned i = 0; i < times; ++i)
+            churnKernel<<<blocks, threads>>>(alloc.getAllocatorHandle(), 20u + i, lo, hi,
+                                             static_cast<const char*>(pool.p), pool.size, d_counts);
+        cudaMemcpy(counts, d_counts, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
+        *hidden = hidden_pages(alloc.getAllocatorHandle().devAllocator);
+        cudaFree(d_counts);
+        return cudaDeviceSynchronize() == cudaSuccess ? 0 : 2;
     }
     catch(const std::exception& e)
     {
