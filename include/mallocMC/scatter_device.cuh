@@ -856,12 +856,14 @@ namespace mmc
             const bool lead = lane == static_cast<u32>(leader);
             const u32 rank = static_cast<u32>(__popc(peers & lanemask_lt()));
             const u32 R = h.regionsize;
-            const u32 region_offset = (start / R) * R;
             const u32 region_ok = __shfl_sync(peers, fill0 < R * 3u / 4u ? 1u : 0u, leader);
             if(region_ok == 0u)
                 return false;
+            /* the leader's start page: the others' may be another, where they
+             * read the first-free-block hint apart and it moved in between */
+            u32 page = __shfl_sync(peers, start, leader);
+            const u32 region_offset = (page / R) * R;
             u32 served = 0u;
-            u32 page = start;
 #pragma unroll 1
             for(u32 visited = 0; visited < R && served < k; ++visited)
             {
